@@ -38,14 +38,6 @@ __device__ __forceinline__ __half half_round_sr(float x, float u) {
     return (x - flo > u * (fhi - flo)) ? hi : lo;
 }
 
-// bf16 stochastic rounding: add 16 random bits below the kept mantissa, then truncate.
-__device__ __forceinline__ uint32_t bf16_round_sr(float x, uint32_t r16) {
-    const uint32_t b = __float_as_uint(x);
-    if ((b & 0x7f800000u) == 0x7f800000u)  // inf / nan: round to nearest
-        return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(x));
-    return (b + r16) >> 16;
-}
-
 template <>
 struct Conv<kHalf> {
     static constexpr int kPairs = 4;  // element pairs per 16-byte word
@@ -76,7 +68,10 @@ struct Conv<kBf16> {
         (&w.x)[h] = *reinterpret_cast<uint32_t *>(&t);
     }
     __device__ __forceinline__ static void put_sr(uint4 &w, int h, float a, float b, uint32_t bits) {
-        (&w.x)[h] = (bf16_round_sr(a, bits & 0xffffu) & 0xffffu) | (bf16_round_sr(b, bits >> 16) << 16);
+        // Adds 16 random bits below the kept mantissa (the low half of `bits` to a, the high half
+        // to b) and truncates; infinities stay, NaN becomes the canonical one.  One instruction
+        // for the pair: checked against (float bits + r16) >> 16 over all 2^32 inputs.
+        asm("cvt.rs.bf16x2.f32 %0, %1, %2, %3;\n" : "=r"((&w.x)[h]) : "f"(b), "f"(a), "r"(bits));
     }
 };
 
