@@ -31,6 +31,7 @@ LIB_SOURCES = [
     "api_io.cpp",
     "api_train.cpp",
     "stream_train.cpp",
+    "scratch.cpp",
     "noalloc.cu",
     "tc_gemm.cu",
     "mlp.cu",

@@ -342,7 +342,7 @@ int train_mode_a(const cumf_problem *tr, const cumf_problem *va, const cumf_para
     int dev = 0, sms = 0;
     CUMF_CUDA(cudaGetDevice(&dev));
     CUMF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const bool one_wave = workers <= resident_workers(k, p.precision, lanes, sms);
+    const bool one_wave = workers <= wave_workers(k, p.precision, lanes, sms);
     int per_launch = (per_epoch || !one_wave || p.tail_epochs > 0 || p.epochs_per_launch <= 0)
                          ? 1
                          : p.epochs_per_launch;
@@ -540,7 +540,7 @@ int cumf_device_info(int gpu, int *sm_count, int *cc_major, int *cc_minor) {
 
 int cumf_default_workers(int sm_count, int k, int precision, int lanes) {
     if (lanes == 0) lanes = default_lanes(k, precision);
-    const int w = resident_workers(k, precision, lanes, sm_count);
+    const int w = wave_workers(k, precision, lanes, sm_count);
     cudaGetLastError();
     return w > 0 ? w : 52 * sm_count;
 }

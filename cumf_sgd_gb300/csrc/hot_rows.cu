@@ -223,7 +223,7 @@ int64_t hot_rows_per_copy(int64_t nnz, int32_t num_workers, int k, int precision
                           int sm_count) {
     if (!(concurrency > 0.f) || nnz <= 0 || num_workers < 2) return 0;
     const int l = lanes > 0 ? lanes : default_lanes(k, precision);
-    const int64_t resident = std::max(1, resident_workers(k, precision, l, sm_count));
+    const int64_t resident = std::max(1, wave_workers(k, precision, l, sm_count));
     const int64_t w = std::min<int64_t>(num_workers, resident);
     // Expected workers on one row at a time = w * count / nnz; a copy carries at most
     // `concurrency` of them, and never fewer than kHotMinPerCopy ratings an epoch.

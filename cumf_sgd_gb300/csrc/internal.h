@@ -51,6 +51,11 @@ inline int64_t batches_per_worker(int64_t nnz, int workers) {
     return (nnz + per - 1) / per;
 }
 
+// ---- scratch.cpp ----------------------------------------------------------------------
+// Stream-ordered device scratch from a pool of the library that keeps up to 256 MB per device
+// between calls; freed with cudaFreeAsync on the stream of its last use.
+cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t s);
+
 // ---- sgd_update.cu -------------------------------------------------------------------
 struct Tuning {
     int lanes = 0;      // 0 = default
@@ -63,8 +68,10 @@ struct Tuning {
 Tuning resolve_tuning(int k, int precision, Tuning t);
 int default_lanes(int k, int precision);
 bool lanes_supported(int k, int precision, int lanes);
-int workers_per_block(int lanes);
+// Workers that fit the GPU at once (the kernel's occupancy), and the workers of one wave of the
+// automatic worker count (1024 threads per SM; 0 without a device or kernel).
 int resident_workers(int k, int precision, int lanes, int sm_count);
+int wave_workers(int k, int precision, int lanes, int sm_count);
 cudaError_t launch_sgd_update(const cumf_node *d_R, int64_t nnz, void *d_P, int32_t m,
                               void *d_Q, int32_t n, int k, int precision, int num_workers,
                               const Tuning &tuning, const float *d_lr, int first_epoch,

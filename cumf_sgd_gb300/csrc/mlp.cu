@@ -18,7 +18,6 @@
 #include <math.h>
 #include <string.h>
 
-#include <mutex>
 #include <string>
 #include <vector>
 
@@ -79,35 +78,6 @@ __global__ void user_qsum_kernel(const cumf_node *R, int64_t nnz, int32_t m, int
             for (int j = lane; j < k; j += 32) atomicAdd(dst + j, c * q[j]);
         }
     }
-}
-
-// Stream-ordered scratch of the feature extraction from a pool of this library that keeps up
-// to 256 MB between calls (the default pool returns its memory at every synchronisation, and
-// mapping it again cost more than the feature kernels at 50,000 users).
-cudaError_t feature_scratch(void **p, size_t bytes, cudaStream_t s) {
-    static std::mutex mu;
-    static cudaMemPool_t pools[64] = {};
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= 64) return cudaMallocAsync(p, bytes, s);
-    cudaMemPool_t pool;
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        if (!pools[dev]) {
-            cudaMemPoolProps props;
-            memset(&props, 0, sizeof(props));
-            props.allocType = cudaMemAllocationTypePinned;
-            props.location.type = cudaMemLocationTypeDevice;
-            props.location.id = dev;
-            if ((e = cudaMemPoolCreate(&pools[dev], &props)) != cudaSuccess) return e;
-            uint64_t keep = 256ull << 20;
-            if ((e = cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess)
-                return e;
-        }
-        pool = pools[dev];
-    }
-    return cudaMallocFromPoolAsync(p, bytes, pool, s);
 }
 
 // Sort keys of the ratings: the user, or m for a rating outside [0, m) x [0, n) (sorted last
@@ -862,7 +832,7 @@ int cumf_user_features(const cumf_node *d_R, int64_t nnz, const float *d_Q, int3
         auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
         const size_t kb = up((size_t)N * 4 + 4), sb = up(((size_t)m + 1) * 8);
         void *buf = nullptr;
-        CUMF_CUDA(feature_scratch(&buf, 4 * kb + sb + up(tmp_bytes), s));
+        CUMF_CUDA(scratch_alloc(&buf, 4 * kb + sb + up(tmp_bytes), s));
         char *p = static_cast<char *>(buf);
         uint32_t *key = reinterpret_cast<uint32_t *>(p), *idx = reinterpret_cast<uint32_t *>(p + kb);
         uint32_t *key2 = reinterpret_cast<uint32_t *>(p + 2 * kb), *idx2 = reinterpret_cast<uint32_t *>(p + 3 * kb);

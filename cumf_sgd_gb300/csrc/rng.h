@@ -52,14 +52,21 @@ constexpr uint64_t kTagSample = 0x5341u;  // batch starts
 constexpr uint64_t kTagRound = 0x5352u;   // stochastic rounding
 // Factor init tags passed by the caller: P = 1, Q = 2.
 
-// Start record of batch `batch` of worker `worker` in epoch `epoch`: uniform on [0, nnz).
-CUMF_HD uint64_t batch_start(uint64_t seed, uint32_t epoch, uint32_t worker, uint32_t batch,
-                             uint64_t nnz) {
+// Sample stream of worker `worker` in epoch `epoch`.
+CUMF_HD uint64_t sample_stream(uint64_t seed, uint32_t epoch, uint32_t worker) {
     uint64_t h = splitmix64(seed ^ (kTagSample << 48));
     h = splitmix64(h + epoch);
-    h = splitmix64(h + worker);
-    h = splitmix64(h + batch);
-    return mulhi64(h, nnz);
+    return splitmix64(h + worker);
+}
+
+// Start record of batch `batch` of a sample stream: uniform on [0, nnz).
+CUMF_HD uint64_t batch_start_of(uint64_t stream, uint32_t batch, uint64_t nnz) {
+    return mulhi64(splitmix64(stream + batch), nnz);
+}
+
+CUMF_HD uint64_t batch_start(uint64_t seed, uint32_t epoch, uint32_t worker, uint32_t batch,
+                             uint64_t nnz) {
+    return batch_start_of(sample_stream(seed, epoch, worker), batch, nnz);
 }
 
 // Key of a factor-init stream (tag 1 = P, 2 = Q).

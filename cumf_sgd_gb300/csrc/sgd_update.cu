@@ -13,13 +13,19 @@
 // whole warp.  Each lane owns E = k/G consecutive elements of a row and moves them with
 // 16-byte ld.global.cg / st.global.cg, so a k=128 fp16 row (256 B) is one vector per lane
 // of a 16-lane group and two workers share a warp.  The dot product is a butterfly of
-// shfl.xor within the group (every lane ends with the same bits).  The rows of record j+1
-// are loaded while record j is reduced and updated (one-deep software pipeline); when
-// record j+1 touches the row record j just wrote, the freshly computed values are forwarded
-// instead, so each worker still applies its records strictly in order.  Records are staged
-// 32 at a time through shared memory (coalesced 4-byte loads of the 12-byte records).
+// shfl.xor within the group (every lane ends with the same bits).  Two kernels:
+//   sgd_pair_kernel     one 16-byte word per lane (every default width but fp32 k = 256): two
+//                       records at a time;
+//   sgd_hogwild_kernel  two or more words per lane: one record at a time, the next one's rows in
+//                       flight.
+// Either way a worker applies its records strictly in order: a row that an earlier record has
+// just written is forwarded to a record whose loads were issued before the store.  Records
+// are staged 32 (narrow groups: 16) at a time through shared memory (4-byte cp.async copies of
+// the 12-byte records).
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <algorithm>
 
 #include "device_common.cuh"
 #include "internal.h"
@@ -30,6 +36,14 @@ namespace {
 
 constexpr int kBlock = 256;   // threads per block
 constexpr int kMinBlocks = 4; // >= 1024 resident threads per SM (<= 64 registers)
+// Threads per block and blocks per SM of sgd_pair_kernel: 1024 threads per SM (64 registers), 896
+// (72 registers) when popular rows are told apart, or 640 (96 registers) in smaller blocks with
+// stochastic rounding.
+constexpr int pair_block(bool sr) { return sr ? 64 : 128; }
+constexpr int pair_min_blocks(bool sr, bool hot) { return sr ? 10 : hot ? 7 : 8; }
+// Threads per SM that a wave of workers stands for (cumf_default_workers): part of the sample
+// schedule through the automatic worker count, so it stays whatever a kernel's occupancy is.
+constexpr int kWaveThreads = 1024;
 constexpr int kDefaultPrefetch = 2;
 constexpr int kDefaultHints = 1;
 constexpr int kDefaultRing = 0;
@@ -54,6 +68,7 @@ struct UpdateArgs {
     int prefetch;   // rows of record j+prefetch are pulled into L2 while record j runs (0 = off)
     int hints;      // 1 = L2 eviction hints (ratings evict_first, factor rows evict_last)
     int freeze_q;   // 1 = item rows are read but never written (user-side fold-in)
+    const uint32_t *hot;  // bit sets of the popular users and items (sample_popular_kernel), or NULL
 };
 
 // Copy of a word the compiler cannot see through: the update phase re-widens the packed
@@ -294,6 +309,344 @@ sgd_hogwild_kernel(const UpdateArgs a) {
 }
 
 
+// ---- two records at a time ----------------------------------------------------------------
+//
+// What bounds an epoch depends on the worker count.  With a few workers (small matrices, fold-in
+// epochs) it is the chain of one record: load, dot, butterfly, update.  Records j and j+1 that
+// share no row are independent, so both chains run interleaved here; a pair that shares a row
+// takes the serial branch, with the same bits either way.  The rows are loaded at the start of
+// their own pair, not a pair ahead: a worker then has two records between load and store, as
+// many as with one record at a time and the next one's rows in flight.  Loading a pair ahead
+// (four records) is faster still (3,000 x 1,200: 0.25 ms) but loses twice the updates on popular
+// rows: 10,000 x 2,000, 0.9M ratings, Zipf 1.0, 20 epochs, test RMSE 0.8069 at 878 workers and
+// 0.905 at 7,904, against 0.8038 and 0.842 as here (0.8030 and 0.841 one record at a time).
+// With the GPU full the epoch is bound by L2 (and, without row copies, by the queues on popular
+// rows): what pays there is fewer instructions per record (no zero fill, no register moves, no
+// forwarding; fp16 and bf16 products accumulate by mixed-precision fma, exact as the widened
+// ones; f32x2 pairs in the update).  1024 threads per SM: with 80 registers and 768 threads an
+// epoch with row copies takes 8.36 ms, 8.25 here.  The random bits of stochastic rounding want
+// 96 registers (0.93 ms with 64, and 0.98 in blocks of 128).
+// Measured per epoch on GB300 against one record at a time: 300 x 120, 20,000 ratings, fp32
+// 0.41 -> 0.23 ms; 3,000 x 1,200, 200,000, fp16 0.56 -> 0.35; 120,047 x 62,501, 12.4M, k = 64,
+// bf16-SR 2.59 -> 0.85 (to 1.12 by cvt.rs); 480,189 x 17,770, 99M, fp16 with row copies
+// 8.63 -> 8.25.
+
+// s += <p, q> over one word, in element order.  A product of two fp16 (bf16) values is exact in
+// fp32, so the mixed-precision fma rounds as the fma of the widened values does.
+template <int KIND>
+__device__ __forceinline__ float dot_word(const uint4 &p, const uint4 &q, float s) {
+    if (KIND == kFloat) {
+        using C = Conv<kFloat>;
+#pragma unroll
+        for (int h = 0; h < C::kPairs; ++h) {
+            const float2 pp = C::get(p, h), qq = C::get(q, h);
+            s = __fmaf_rn(pp.x, qq.x, s);
+            s = __fmaf_rn(pp.y, qq.y, s);
+        }
+        return s;
+    }
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+        const uint32_t a = (&p.x)[h], b = (&q.x)[h];
+        if (KIND == kHalf)
+            asm("{.reg .f16 x, y, z, w; mov.b32 {x, y}, %1; mov.b32 {z, w}, %2;\n"
+                " fma.rn.f32.f16 %0, x, z, %0; fma.rn.f32.f16 %0, y, w, %0;}\n"
+                : "+f"(s)
+                : "r"(a), "r"(b));
+        else
+            asm("{.reg .b16 x, y, z, w; mov.b32 {x, y}, %1; mov.b32 {z, w}, %2;\n"
+                " fma.rn.f32.bf16 %0, x, z, %0; fma.rn.f32.bf16 %0, y, w, %0;}\n"
+                : "+f"(s)
+                : "r"(a), "r"(b));
+    }
+    return s;
+}
+
+__device__ __forceinline__ float2 both(float x) { return make_float2(x, x); }
+
+// update_rows for one word, two elements per instruction; nlp = -lambda_p, nlq = -lambda_q
+// (-(l*x) and (-l)*x are the same bits).
+template <int KIND, bool SR>
+__device__ __forceinline__ void update_word(const uint4 &p, const uint4 &q, uint4 &wp, uint4 &wq, float lr, float err,
+                                            float nlp, float nlq, uint32_t key, int lane) {
+    using C = Conv<KIND>;
+#pragma unroll
+    for (int h = 0; h < C::kPairs; ++h) {
+        const float2 pp = C::get(p, h), qq = C::get(q, h);
+        const float2 a = __ffma2_rn(both(lr), __ffma2_rn(both(err), qq, __fmul2_rn(both(nlp), pp)), pp);
+        const float2 b = __ffma2_rn(both(lr), __ffma2_rn(both(err), pp, __fmul2_rn(both(nlq), qq)), qq);
+        if (SR) {
+            const uint32_t pair = (uint32_t)((lane * C::kPairs + h) * 2);
+            C::put_sr(wp, h, a.x, a.y, lowbias32(key + pair));
+            C::put_sr(wq, h, b.x, b.y, lowbias32(key + pair + 1u));
+        } else {
+            C::put(wp, h, a.x, a.y);
+            C::put(wq, h, b.x, b.y);
+        }
+    }
+}
+
+// ---- popular rows -------------------------------------------------------------------------
+//
+// A row that many workers hold at once is bound by its cache lines: every store takes the line
+// from the SMs that read it, and the next load fetches it back, about 150 ns a turn.  A 16-byte
+// atomic exchange writes at the line's home in L2 instead and spares the turns.  Measured,
+// random read-modify-writes of H rows of 256 bytes by 9,728 workers, ns per row, store /
+// exchange: H = 8 3.6 / 2.6, 64 1.05 / 0.46, 512 0.31 / 0.17, 17,770 0.060 / 0.080.  So rows
+// that about kPopularWorkers records in flight name at a time are written by exchange (the same
+// bits either way), the others by plain stores.  Per epoch, with all stores plain / this rule:
+// 480,189 x 17,770, 99M ratings, fp16 14.2 / 10.4 ms (60 items, 4% of the ratings; at 4 workers
+// 10.3, at 2 10.6, every row 16.5); 10,000 x 2,000, 0.9M, Zipf 1.0 2.55 / 0.83; 240,000 x
+// 17,770, 50M, fp32 10.0 / 9.2.
+// Which rows those are is sampled before the launch: up to 2 ratings per record in flight are
+// counted by hashed id, and the ids whose count reaches the limit form two bit sets that the
+// update kernel keeps in shared memory.  The bits only choose the store instruction: a wrong one
+// costs time, never a result.  With few records in flight the exchanges' own latency costs more
+// than the turns: fp16, Zipf 1.0 as above, 256 workers 1.85 ms plain, 1.9-2.1 by exchange, 512
+// workers 2.36, 1.12; 3,000 x 1,200 at 390 records in flight 0.36 plain, 0.42 with the rule; and
+// the longer chains of stochastic rounding queue later (30,000 x 6,000, k = 64, bf16-SR, 878
+// workers 1.8 plain, 2.25 by exchange; 2,048 workers 1.83, 1.12).
+constexpr int kPopularBits = 14;  // hashed ids per side: 16,384 (unpopular ids share few hits)
+constexpr int kPopularWords = (1 << kPopularBits) / 32;
+constexpr int kPopularWorkers = 8;
+constexpr int kSampleThreads = 1024;
+constexpr int kMaxSamples = 16384;
+
+__device__ __forceinline__ uint32_t popular_hash(uint32_t id) { return (id * 0x9E3779B1u) >> (32 - kPopularBits); }
+
+constexpr int popular_min_in_flight(bool sr) { return sr ? 4096 : 1024; }
+
+// Block 0: users, block 1: items.  `samples` < 2^16 (16-bit counters, two to a word).
+__global__ void __launch_bounds__(kSampleThreads) sample_popular_kernel(const cumf_node *R, uint64_t nnz, uint32_t m,
+                                                                        uint32_t n, int samples, uint32_t limit,
+                                                                        uint64_t key, uint32_t *bits) {
+    __shared__ uint32_t cnt[(1 << kPopularBits) / 2];
+    for (int i = threadIdx.x; i < (1 << kPopularBits) / 2; i += kSampleThreads) cnt[i] = 0;
+    __syncthreads();
+    const uint32_t rows = blockIdx.x == 0 ? m : n;
+    const uint32_t *const ids = reinterpret_cast<const uint32_t *>(R) + blockIdx.x;
+#pragma unroll 8
+    for (int i = threadIdx.x; i < samples; i += kSampleThreads) {
+        const uint32_t id = __ldg(ids + 3 * mulhi64(splitmix64(key + (uint64_t)i), nnz));
+        if (id < rows) {
+            const uint32_t h = popular_hash(id);
+            atomicAdd(&cnt[h >> 1], 1u << ((h & 1) * 16));
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < kPopularWords) {
+        uint32_t w = 0;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const uint32_t c = cnt[threadIdx.x * 16 + i];
+            w |= (uint32_t)((c & 0xffffu) >= limit) << (2 * i) | (uint32_t)((c >> 16) >= limit) << (2 * i + 1);
+        }
+        bits[blockIdx.x * kPopularWords + threadIdx.x] = w;
+    }
+}
+
+__device__ __forceinline__ void store_row(uint4 *p, uint4 v, uint64_t pol, uint32_t popular) {
+    if (popular) {
+        const uint64_t lo = (uint64_t)v.x | ((uint64_t)v.y << 32), hi = (uint64_t)v.z | ((uint64_t)v.w << 32);
+        asm volatile("{.reg .b128 x, y; mov.b128 x, {%1, %2}; atom.relaxed.gpu.global.exch.b128 y, [%0], x;}\n" ::"l"(p),
+                     "l"(lo), "l"(hi)
+                     : "memory");
+    } else {
+        st_row_hint(p, v, pol);
+    }
+}
+
+// HOT: the launch has popular rows to tell apart (a.hot); item rows are not frozen.
+template <int K, int KIND, int G, bool SR, bool HOT>
+__global__ void __launch_bounds__(pair_block(SR), pair_min_blocks(SR, HOT)) sgd_pair_kernel(const UpdateArgs a) {
+    constexpr int ROW_WORDS = K * store_bytes(KIND) / 16;
+    static_assert(ROW_WORDS == G, "one word per lane");
+    constexpr int kChunk = chunk_of(G);
+    constexpr int CPB = kBatch / kChunk;
+    constexpr int CW = kChunk * 3;  // words of a staged chunk
+    constexpr int WPL = CW / G;
+    static_assert(CW % G == 0 && kBatch % kChunk == 0 && kChunk % 2 == 0, "chunk must split evenly");
+    // Two chunks per group, records as they are in memory; the odd stride keeps the groups of a
+    // warp on different banks.
+    __shared__ uint32_t s_rec[pair_block(SR) / G][2 * CW + 1];
+    __shared__ uint32_t s_popular[2][HOT ? kPopularWords : 1];  // users, items
+    int any_popular = 0;
+    if (HOT) {
+        for (int i = threadIdx.x; i < 2 * kPopularWords; i += pair_block(SR)) {
+            const uint32_t w = __ldg(a.hot + i);
+            (&s_popular[0][0])[i] = w;
+            any_popular |= w != 0;
+        }
+        any_popular = __syncthreads_or(any_popular);
+    }
+
+    const int lane = threadIdx.x % G;
+    const int worker = blockIdx.x * (pair_block(SR) / G) + threadIdx.x / G;
+    if (worker >= a.num_workers) return;
+    const unsigned gmask =
+        (G == 32) ? 0xffffffffu : (((1u << G) - 1u) << ((threadIdx.x & 31) & ~(G - 1)));
+    uint4 *const P = reinterpret_cast<uint4 *>(a.P) + lane;
+    uint4 *const Q = reinterpret_cast<uint4 *>(a.Q) + lane;
+    const uint32_t *const Rw = reinterpret_cast<const uint32_t *>(a.R);
+    uint32_t *const rec = s_rec[threadIdx.x / G];
+    const uint64_t nnz = a.nnz;
+    const uint32_t m1 = a.m - 1, n1 = a.n - 1;
+    const float nlp = -a.lambda_p, nlq = -a.lambda_q;
+    const int chunks = a.batches * CPB;
+    const uint32_t x0 = (uint32_t)worker * (uint32_t)(chunks * kChunk);  // sample index of the first record
+    const uint64_t pol_rec = l2_policy(a.hints != 0, false);
+    const uint64_t pol_row = l2_policy(a.hints != 0, true);
+    const bool pf_lane = a.prefetch > 0 && (lane & 7) == 0;  // lanes that start a 128-byte line
+    int bad = 0;
+
+    for (int ep = a.first_epoch; ep < a.first_epoch + a.n_epochs; ++ep) {
+        const float lr = __ldg(a.lr + ep);
+        const uint32_t round_key = (uint32_t)(splitmix64(a.seed ^ (kTagRound << 48)) + (uint64_t)ep);
+        const uint64_t stream = sample_stream(a.seed, ep, worker);
+
+        // Asynchronous copy of the records of chunk t into half t & 1 of the ring.
+        auto fetch = [&](int t) {
+            uint64_t base = batch_start_of(stream, t / CPB, nnz) + (uint64_t)((t % CPB) * kChunk);
+            while (base >= nnz) base -= nnz;  // start < nnz: wraps more than once only when nnz < 128
+            uint32_t *dst = rec + (t & 1) * CW + lane;
+            if (base + kChunk <= nnz) {
+                const uint32_t *src = Rw + base * 3 + lane;
+#pragma unroll
+                for (int i = 0; i < WPL; ++i) cp_async4(dst + i * G, src + i * G, pol_rec);
+            } else {
+                for (int i = 0; i < WPL; ++i) {
+                    const int word = lane + i * G;
+                    uint64_t r = base + (uint64_t)(word / 3);
+                    while (r >= nnz) r -= nnz;
+                    cp_async4(dst + i * G, Rw + r * 3 + (word % 3), pol_rec);
+                }
+            }
+            cp_async_commit();
+        };
+        __syncwarp(gmask);  // the last epoch's records are no longer read
+        fetch(0);
+        cp_async_wait_all();
+        __syncwarp(gmask);
+
+        // Bit j of hp (hq): the user (item) of record j of chunk t is popular.
+        auto popular = [&](int t, uint32_t &hp, uint32_t &hq) {
+            hp = hq = 0;
+            if (!HOT || !any_popular) return;
+            const int shift = threadIdx.x & 31 & ~(G - 1);
+            const uint32_t group = (G == 32) ? 0xffffffffu : (1u << G) - 1u;
+#pragma unroll
+            for (int i = 0; i < kChunk / G; ++i) {
+                const uint32_t *w = rec + (t & 1) * CW + 3 * (lane + i * G);
+                const uint32_t h = popular_hash(w[0]), g = popular_hash(w[1]);
+                hp |= ((__ballot_sync(gmask, (s_popular[0][h >> 5] >> (h & 31)) & 1u) >> shift) & group) << (i * G);
+                hq |= ((__ballot_sync(gmask, (s_popular[1][g >> 5] >> (g & 31)) & 1u) >> shift) & group) << (i * G);
+            }
+        };
+        // One record on its own: rows p and q become the updated ones, and are stored.
+        auto apply = [&](uint4 &p, uint4 &q, uint32_t uu, uint32_t vv, float r, uint32_t x, uint32_t hu, uint32_t hv) {
+            float s = dot_word<KIND>(p, q, 0.f);
+#pragma unroll
+            for (int o = G / 2; o >= 1; o >>= 1) s += __shfl_xor_sync(gmask, s, o);
+            uint4 wp, wq;
+            update_word<KIND, SR>(p, q, wp, wq, lr, r - s, nlp, nlq, SR ? round_key ^ lowbias32(x) : 0u, lane);
+            p = wp;
+            store_row(P + (uint64_t)uu * ROW_WORDS, p, pol_row, hu);
+            if (HOT || !a.freeze_q) {
+                q = wq;
+                store_row(Q + (uint64_t)vv * ROW_WORDS, q, pol_row, hv);
+            }
+        };
+        uint32_t nu[2], nv[2];  // ids of the next pair
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            nu[e] = rec[3 * e];
+            nv[e] = rec[3 * e + 1];
+        }
+        uint32_t hp, hq;
+        popular(0, hp, hq);
+
+        for (int t = 0; t < chunks; ++t) {
+            __syncwarp(gmask);  // the half refilled next is no longer read
+            if (t + 1 < chunks) fetch(t + 1);
+            const uint32_t *cur = rec + (t & 1) * CW;
+            const int next_half = (t & 1) ? -2 * CW : 0;  // added to an index past this chunk's end
+
+#pragma unroll 1
+            for (int j = 0; j < kChunk; j += 2, hp >>= 2, hq >>= 2) {
+                const uint32_t ua = nu[0], ub = nu[1], va = nv[0], vb = nv[1];
+                // Ids outside the matrices load the last row instead; such records are not applied.
+                uint4 *const pa = P + (uint64_t)min(ua, m1) * ROW_WORDS, *const qa = Q + (uint64_t)min(va, n1) * ROW_WORDS;
+                uint4 *const pb = P + (uint64_t)min(ub, m1) * ROW_WORDS, *const qb = Q + (uint64_t)min(vb, n1) * ROW_WORDS;
+                uint4 fpa = ld_row_hint(pa, pol_row), fqa = ld_row_hint(qa, pol_row);
+                uint4 fpb = ld_row_hint(pb, pol_row), fqb = ld_row_hint(qb, pol_row);
+                if (j == kChunk - 2) {  // the look-ahead enters the next chunk
+                    cp_async_wait_all();
+                    __syncwarp(gmask);
+                }
+                // (Past the last chunk this reads old records' ids, which are not used.)
+                const uint32_t *ahead = cur + 3 * (j + 2) + (j + 2 >= kChunk ? next_half : 0);
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    nu[e] = ahead[3 * e];
+                    nv[e] = ahead[3 * e + 1];
+                }
+                if (pf_lane) {
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        prefetch_l2(P + (uint64_t)min(nu[e], m1) * ROW_WORDS);
+                        prefetch_l2(Q + (uint64_t)min(nv[e], n1) * ROW_WORDS);
+                    }
+                }
+                const bool oka = (ua <= m1) & (va <= n1), okb = (ub <= m1) & (vb <= n1);
+                const float ra = __uint_as_float(cur[3 * j + 2]), rb = __uint_as_float(cur[3 * j + 5]);
+                const uint32_t x = x0 + (uint32_t)(t * kChunk + j);
+                if (__builtin_expect(oka & okb & (ua != ub) & (va != vb), 1)) {
+                    float sa = dot_word<KIND>(fpa, fqa, 0.f), sb = dot_word<KIND>(fpb, fqb, 0.f);
+#pragma unroll
+                    for (int o = G / 2; o >= 1; o >>= 1) {
+                        sa += __shfl_xor_sync(gmask, sa, o);
+                        sb += __shfl_xor_sync(gmask, sb, o);
+                    }
+                    uint4 wpa, wqa, wpb, wqb;
+                    update_word<KIND, SR>(fpa, fqa, wpa, wqa, lr, ra - sa, nlp, nlq, SR ? round_key ^ lowbias32(x) : 0u,
+                                          lane);
+                    if (!HOT) {
+                        st_row_hint(pa, wpa, pol_row);
+                        if (!a.freeze_q) st_row_hint(qa, wqa, pol_row);
+                    }
+                    update_word<KIND, SR>(fpb, fqb, wpb, wqb, lr, rb - sb, nlp, nlq,
+                                          SR ? round_key ^ lowbias32(x + 1u) : 0u, lane);
+                    if (!HOT) {
+                        st_row_hint(pb, wpb, pol_row);
+                        if (!a.freeze_q) st_row_hint(qb, wqb, pol_row);
+                    } else if (__builtin_expect(((hp | hq) & 3u) == 0, 1)) {
+                        st_row_hint(pa, wpa, pol_row);
+                        st_row_hint(qa, wqa, pol_row);
+                        st_row_hint(pb, wpb, pol_row);
+                        st_row_hint(qb, wqb, pol_row);
+                    } else {
+                        store_row(pa, wpa, pol_row, hp & 1u);
+                        store_row(qa, wqa, pol_row, hq & 1u);
+                        store_row(pb, wpb, pol_row, hp & 2u);
+                        store_row(qb, wqb, pol_row, hq & 2u);
+                    }
+                } else {
+                    if (oka) {
+                        apply(fpa, fqa, ua, va, ra, x, hp & 1u, hq & 1u);
+                        if (ub == ua) fpb = fpa;
+                        if (vb == va) fqb = fqa;
+                    }
+                    if (okb) apply(fpb, fqb, ub, vb, rb, x + 1u, hp & 2u, hq & 2u);
+                    if (!(oka & okb)) bad = 1;
+                }
+            }
+            popular(t + 1, hp, hq);  // (past the last chunk: old records, not used)
+        }
+    }
+    if (bad && a.status != nullptr && lane == 0) atomicExch(a.status, (int)CUMF_ERR_RANGE);
+}
+
+
 // ---- deeper pipeline: rows staged asynchronously through a shared-memory ring ----------
 //
 // Same semantics as sgd_hogwild_kernel, with D records' rows in flight per worker instead
@@ -492,13 +845,21 @@ using KernelFn = void (*)(const UpdateArgs);
 struct KernelEntry {
     int k, kind, lanes;
     bool sr;
-    KernelFn fn;
+    KernelFn fn;          // sgd_pair_kernel, or sgd_hogwild_kernel where a lane holds several words
+    KernelFn hot;         // sgd_pair_kernel with popular rows told apart (nullptr otherwise)
     KernelFn ring;        // deeper-pipeline variant (nullptr where not built)
     size_t ring_smem;     // its dynamic shared memory per block
 };
 
-#define CUMF_K(K, KIND, G, SR) {K, KIND, G, SR, &sgd_hogwild_kernel<K, KIND, G, SR>, \
-    &sgd_ring_kernel<K, KIND, G, SR, kRingDepth>, RingLayout<K, KIND, G, kRingDepth>::smem}
+// The kernel of a lane width: two records at a time where a lane holds one 16-byte word of a row.
+template <int K, int KIND, int G, bool SR, bool HOT>
+constexpr KernelFn update_kernel() {
+    if constexpr (K * store_bytes(KIND) / 16 == G) return &sgd_pair_kernel<K, KIND, G, SR, HOT>;
+    else return HOT ? nullptr : &sgd_hogwild_kernel<K, KIND, G, SR>;
+}
+
+#define CUMF_K(K, KIND, G, SR) {K, KIND, G, SR, update_kernel<K, KIND, G, SR, false>(), \
+    update_kernel<K, KIND, G, SR, true>(), &sgd_ring_kernel<K, KIND, G, SR, kRingDepth>, RingLayout<K, KIND, G, kRingDepth>::smem}
 #define CUMF_K_ALL_G(K, KIND, SR, G1, G2) CUMF_K(K, KIND, G1, SR), CUMF_K(K, KIND, G2, SR)
 
 // For each (k, storage) two lane widths: one 16-byte word per lane, or two.
@@ -555,29 +916,25 @@ bool lanes_supported(int k, int precision, int lanes) {
     return find_kernel(k, precision, lanes) != nullptr;
 }
 
-int workers_per_block(int lanes) { return kBlock / lanes; }
-
 // The ring kernels need more than the default 48 KB of dynamic shared memory.
-cudaError_t prepare_ring(const KernelEntry *e) {
+static cudaError_t prepare_ring(const KernelEntry *e) {
     return cudaFuncSetAttribute(e->ring, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->ring_smem);
-}
-
-int resident_workers_of(const KernelEntry *e, bool ring, int sm_count) {
-    int blocks = 0;
-    if (ring) {
-        if (prepare_ring(e) != cudaSuccess) return 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, e->ring, kBlock, e->ring_smem) != cudaSuccess)
-            return 0;
-    } else if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, e->fn, kBlock, 0) != cudaSuccess) {
-        return 0;
-    }
-    return blocks * sm_count * (kBlock / e->lanes);
 }
 
 int resident_workers(int k, int precision, int lanes, int sm_count) {
     const KernelEntry *e = find_kernel(k, precision, lanes);
     if (!e) return 0;
-    return resident_workers_of(e, kDefaultRing != 0, sm_count);
+    const int threads = e->hot ? pair_block(e->sr) : kBlock;
+    int blocks = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, e->fn, threads, 0) != cudaSuccess) return 0;
+    return blocks * sm_count * (threads / e->lanes);
+}
+
+int wave_workers(int k, int precision, int lanes, int sm_count) {
+    const KernelEntry *e = find_kernel(k, precision, lanes);
+    int devices = 0;
+    if (!e || cudaGetDeviceCount(&devices) != cudaSuccess || devices <= 0) return 0;
+    return kWaveThreads / e->lanes * sm_count;
 }
 
 // With the hot rows split into copies, or with the item rows frozen (fold-in epochs), no
@@ -587,12 +944,7 @@ int resident_workers(int k, int precision, int lanes, int sm_count) {
 // 5.2M-rating fold-in epoch: fp16 0.76 against 0.85 ms, bf16-SR 1.31 against 1.37); with
 // factors far beyond L2 the row loads go to DRAM and the prefetch pays again (c3, 1,000,990 x
 // 624,961, 416 MB of fp16 factors: 28.2 ms with it against 31.4 without).
-static int copies_prefetch(int32_t m, int32_t n, int k, int precision) {
-    int dev = 0, l2 = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess) {
-        cudaGetLastError();
-        l2 = 126 << 20;
-    }
+static int copies_prefetch(int32_t m, int32_t n, int k, int precision, int l2) {
     const double bytes = ((double)m + (double)n) * k * elem_bytes(precision);
     return bytes > 2.0 * l2 ? kDefaultPrefetch : 0;
 }
@@ -612,9 +964,16 @@ cudaError_t launch_sgd_update(const cumf_node *d_R, int64_t nnz, void *d_P, int3
                               int n_epochs, float lambda_p, float lambda_q, uint64_t seed,
                               int *d_status, cudaStream_t stream, int *lanes_used) {
     Tuning t = resolve_tuning(k, precision, tuning);
-    if (tuning.prefetch < 0 && (tuning.copies || tuning.freeze_q)) t.prefetch = copies_prefetch(m, n, k, precision);
+    int dev = 0, l2 = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+        cudaGetLastError();
+        l2 = 126 << 20;
+        sms = 152;
+    }
     const KernelEntry *e = find_kernel(k, precision, t.lanes);
     if (!e) return cudaErrorInvalidValue;
+    if (tuning.prefetch < 0 && (tuning.copies || tuning.freeze_q)) t.prefetch = copies_prefetch(m, n, k, precision, l2);
     if (lanes_used) *lanes_used = e->lanes;
     if (nnz <= 0 || n_epochs <= 0 || num_workers <= 0) return cudaSuccess;
     UpdateArgs a;
@@ -636,16 +995,53 @@ cudaError_t launch_sgd_update(const cumf_node *d_R, int64_t nnz, void *d_P, int3
     a.prefetch = t.prefetch;
     a.hints = t.hints;
     a.freeze_q = t.freeze_q;
-    const int gpb = kBlock / e->lanes;
-    const int blocks = (num_workers + gpb - 1) / gpb;
+    a.hot = nullptr;
+    // Every worker has to run an epoch before any runs the next one's learning rate: with more
+    // workers than fit, one launch per epoch.
+    if (n_epochs > 1 && !t.ring && num_workers > resident_workers(k, precision, e->lanes, sms)) {
+        for (int ep = first_epoch; ep < first_epoch + n_epochs; ++ep) {
+            const cudaError_t ce = launch_sgd_update(d_R, nnz, d_P, m, d_Q, n, k, precision, num_workers, tuning, d_lr, ep,
+                                                     1, lambda_p, lambda_q, seed, d_status, stream, nullptr);
+            if (ce != cudaSuccess) return ce;
+        }
+        return cudaSuccess;
+    }
     if (t.ring) {
         cudaError_t ce = prepare_ring(e);
         if (ce != cudaSuccess) return ce;
-        e->ring<<<blocks, kBlock, e->ring_smem, stream>>>(a);
-    } else {
-        e->fn<<<blocks, kBlock, 0, stream>>>(a);
+        const int gpb = kBlock / e->lanes;
+        e->ring<<<(num_workers + gpb - 1) / gpb, kBlock, e->ring_smem, stream>>>(a);
+        return cudaGetLastError();
     }
-    return cudaGetLastError();
+    const int threads = e->hot ? pair_block(e->sr) : kBlock, gpb = threads / e->lanes;
+    // Row copies have no popular rows, and frozen item rows are not stored.  Under stream capture
+    // (and when no scratch can be had) every store is plain.
+    void *popular = nullptr;
+    const int64_t in_flight = 2ll * std::min(num_workers, threads * pair_min_blocks(e->sr, true) / e->lanes * sms);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (e->hot && !tuning.copies && !t.freeze_q && in_flight >= popular_min_in_flight(e->sr)) {
+        if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
+            scratch_alloc(&popular, 2 * kPopularWords * sizeof(uint32_t), stream) != cudaSuccess) {
+            cudaGetLastError();
+            popular = nullptr;
+        }
+    }
+    if (popular) {
+        const int samples = (int)std::min<int64_t>(2 * in_flight, kMaxSamples);
+        // Well above the hits of the unpopular ids that share a hashed id, too.
+        const int64_t limit = std::max<int64_t>((int64_t)kPopularWorkers * samples / in_flight,
+                                                2 + 4ll * samples / (1 << kPopularBits));
+        sample_popular_kernel<<<2, kSampleThreads, 0, stream>>>(d_R, a.nnz, a.m, a.n, samples, (uint32_t)limit,
+                                                                splitmix64(seed), static_cast<uint32_t *>(popular));
+    }
+    a.hot = static_cast<const uint32_t *>(popular);
+    (popular ? e->hot : e->fn)<<<(num_workers + gpb - 1) / gpb, threads, 0, stream>>>(a);
+    cudaError_t ce = cudaGetLastError();
+    if (popular) {
+        const cudaError_t ef = cudaFreeAsync(popular, stream);
+        if (ce == cudaSuccess) ce = ef;
+    }
+    return ce;
 }
 
 }  // namespace cumf
