@@ -55,158 +55,211 @@ struct BatchTask {
     int worker;
 };
 
-// A lane's slice of a row: E consecutive halves moved as NVEC vectors of type V.
-template <int E>
-struct LaneIO;
-template <>
-struct LaneIO<2> {
-    using V = uint32_t;
-    static constexpr int NVEC = 1;
-};
-template <>
-struct LaneIO<4> {
-    using V = uint2;
-    static constexpr int NVEC = 1;
-};
-template <>
-struct LaneIO<8> {
-    using V = uint4;
-    static constexpr int NVEC = 1;
-};
-template <>
-struct LaneIO<16> {
-    using V = uint4;
-    static constexpr int NVEC = 2;
-};
-
-template <typename T>
-__device__ __forceinline__ uint32_t &word(T &v, int w) {
-    return reinterpret_cast<uint32_t *>(&v)[w];
-}
-
 __device__ __forceinline__ void bcp_async4(void *smem, const void *gmem) {
     const uint32_t sa = (uint32_t)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa), "l"(gmem) : "memory");
 }
 
-// One worker's epoch on one problem: G lanes, E = k / G halves per lane (the lane's slice
-// starts at element lane * E).  Dot product: lane partial in element order, then a shfl.xor
-// butterfly over the G lanes (the order the oracle replays with lanes = G).
-template <int G, int E>
-__device__ void run_task(const BatchProblemDev &pr, int worker, int ep, int lane, unsigned gmask,
-                         uint32_t (*s_rec)[3][kBChunk + 1], int *bad) {
-    using IO = LaneIO<E>;
-    using V = typename IO::V;
-    constexpr int NVEC = IO::NVEC;
-    constexpr int WPV = (int)(sizeof(V) / 4);  // 32-bit words (half pairs) per vector
-    constexpr int ROWV = G * NVEC;             // vectors per row
-    constexpr int WPL = kBChunk * 3 / G;       // staged record words per lane
-    static_assert((kBChunk * 3) % G == 0, "record staging must split over the lanes");
-    V *const P = reinterpret_cast<V *>(pr.P) + lane * NVEC;
-    V *const Q = reinterpret_cast<V *>(pr.Q) + lane * NVEC;
+// ---- two records at a time ----------------------------------------------------------------
+//
+// A worker is a group of G lanes and a row is G slices of SB bytes (k / G halves); a dot product
+// adds the slices' partial sums in a butterfly over G (the order that the oracle replays with
+// lanes = G).  Records j and j+1 that share no row are independent: the low half of the lanes
+// takes record j, the high half record j+1, each lane two slices of its record, hl and hl + G/2,
+// so the butterfly's first step is an addition within the lane.  With rows of 64 to 256 bytes the
+// kernel was bound by instructions per record, and this nearly halves those for ids, addresses
+// and shuffles.  A pair that shares a row or names one outside the matrices goes one record after
+// the other, with the same bits.  The lanes of a worker see each other's stores through the
+// __syncwarp that begins every pair.
+template <int SB>
+struct Slice {
+    uint32_t w[SB / 4];
+};
+
+template <int SB>
+__device__ __forceinline__ void load_slice(Slice<SB> &s, const char *p) {
+    if constexpr (SB == 4) {
+        s.w[0] = __ldcg(reinterpret_cast<const uint32_t *>(p));
+    } else if constexpr (SB == 8) {
+        const uint2 v = __ldcg(reinterpret_cast<const uint2 *>(p));
+        s.w[0] = v.x;
+        s.w[1] = v.y;
+    } else {
+#pragma unroll
+        for (int i = 0; i < SB / 16; ++i) {
+            const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(p) + i);
+            s.w[4 * i] = v.x;
+            s.w[4 * i + 1] = v.y;
+            s.w[4 * i + 2] = v.z;
+            s.w[4 * i + 3] = v.w;
+        }
+    }
+}
+
+template <int SB>
+__device__ __forceinline__ void store_slice(char *p, const Slice<SB> &s) {
+    if constexpr (SB == 4) {
+        __stcg(reinterpret_cast<uint32_t *>(p), s.w[0]);
+    } else if constexpr (SB == 8) {
+        __stcg(reinterpret_cast<uint2 *>(p), make_uint2(s.w[0], s.w[1]));
+    } else {
+#pragma unroll
+        for (int i = 0; i < SB / 16; ++i)
+            __stcg(reinterpret_cast<uint4 *>(p) + i,
+                   make_uint4(s.w[4 * i], s.w[4 * i + 1], s.w[4 * i + 2], s.w[4 * i + 3]));
+    }
+}
+
+__device__ __forceinline__ float2 widen(uint32_t w) { return __half22float2(*reinterpret_cast<__half2 *>(&w)); }
+__device__ __forceinline__ float2 both(float x) { return make_float2(x, x); }
+
+// <p, q> over one slice, in element order.  A product of two fp16 values is exact in fp32, so the
+// mixed-precision fma rounds as the fma of the widened values does.
+template <int SB>
+__device__ __forceinline__ float dot_slice(const Slice<SB> &p, const Slice<SB> &q) {
+    float s = 0.f;
+#pragma unroll
+    for (int h = 0; h < SB / 4; ++h)
+        asm("{.reg .f16 x, y, z, w; mov.b32 {x, y}, %1; mov.b32 {z, w}, %2;\n"
+            " fma.rn.f32.f16 %0, x, z, %0; fma.rn.f32.f16 %0, y, w, %0;}\n"
+            : "+f"(s)
+            : "r"(p.w[h]), "r"(q.w[h]));
+    return s;
+}
+
+// p + lr*(e*q - lp*p) and q + lr*(e*p_old - lq*q) (warp32.h:89-99), two elements per instruction;
+// nlp = -lambda_p, nlq = -lambda_q (-(l*x) and (-l)*x are the same bits).
+template <int SB>
+__device__ __forceinline__ void update_slice(Slice<SB> &p, Slice<SB> &q, float lr, float err, float nlp, float nlq) {
+#pragma unroll
+    for (int h = 0; h < SB / 4; ++h) {
+        const float2 pp = widen(p.w[h]), qq = widen(q.w[h]);
+        const float2 a = __ffma2_rn(both(lr), __ffma2_rn(both(err), qq, __fmul2_rn(both(nlp), pp)), pp);
+        const float2 b = __ffma2_rn(both(lr), __ffma2_rn(both(err), pp, __fmul2_rn(both(nlq), qq)), qq);
+        const __half2 ha = __floats2half2_rn(a.x, a.y), hb = __floats2half2_rn(b.x, b.y);
+        p.w[h] = *reinterpret_cast<const uint32_t *>(&ha);
+        q.w[h] = *reinterpret_cast<const uint32_t *>(&hb);
+    }
+}
+
+// What a lane keeps through a task.
+struct PairLane {
+    char *P, *Q;  // factor matrices at the lane's first slice
+    float lr, nlp, nlq;
+    int hl;       // lane within its half of the group
+};
+
+// One record on the G/2 lanes of `mask` (one half of the group, or both with a record each).
+template <int G, int SB>
+__device__ __forceinline__ void pair_record(const PairLane &c, unsigned mask, uint32_t u, uint32_t v, float r) {
+    constexpr int H = G / 2;
+    char *const p = c.P + (uint64_t)u * (G * SB), *const q = c.Q + (uint64_t)v * (G * SB);
+    Slice<SB> p0, p1, q0, q1;
+    load_slice(p0, p);
+    load_slice(q0, q);
+    load_slice(p1, p + H * SB);
+    load_slice(q1, q + H * SB);
+    float s = dot_slice(p0, q0) + dot_slice(p1, q1);
+#pragma unroll
+    for (int o = H / 2; o >= 1; o >>= 1) s += __shfl_xor_sync(mask, s, o);
+    const float err = r - s;
+    update_slice(p0, q0, c.lr, err, c.nlp, c.nlq);
+    update_slice(p1, q1, c.lr, err, c.nlp, c.nlq);
+    store_slice(p, p0);
+    store_slice(p + H * SB, p1);
+    store_slice(q, q0);
+    store_slice(q + H * SB, q1);
+}
+
+// One worker's epoch on one problem.
+template <int G, int SB>
+__device__ void run_task(const BatchProblemDev &pr, int worker, int ep, int lane, unsigned gmask, uint32_t *rec,
+                         int *bad) {
+    constexpr int H = G / 2;
+    constexpr int CW = kBChunk * 3;       // words of a staged chunk
+    constexpr int WPL = CW / G;
+    constexpr int CPB = 128 / kBChunk;    // chunks per batch
+    static_assert(CW % G == 0, "record staging must split over the lanes");
+    const int half = lane / H;
+    const int shift = threadIdx.x & 31 & ~(G - 1);
+    const uint32_t group = (G == 32) ? 0xffffffffu : (1u << G) - 1u;
+    PairLane c;
+    c.hl = lane % H;
+    c.P = static_cast<char *>(pr.P) + c.hl * SB;
+    c.Q = static_cast<char *>(pr.Q) + c.hl * SB;
+    c.lr = __ldg(pr.lr + ep);
+    c.nlp = -pr.lp;
+    c.nlq = -pr.lq;
     const uint32_t *const Rw = reinterpret_cast<const uint32_t *>(pr.R);
     const uint64_t nnz = pr.nnz;
-    const float lr = __ldg(pr.lr + ep);
-    const int chunks = pr.batches * (128 / kBChunk);
-    auto fetch = [&](int t, int buf) {
-        const uint64_t start = batch_start(pr.seed, ep, worker, t / (128 / kBChunk), nnz);
-        uint64_t base = start + (uint64_t)((t % (128 / kBChunk)) * kBChunk);
-        while (base >= nnz) base -= nnz;
+    const uint32_t m1 = pr.m - 1, n1 = pr.n - 1;
+    const int chunks = pr.batches * CPB;
+    const uint64_t stream = sample_stream(pr.seed, ep, worker);
+    // Asynchronous copy of the records of chunk t into half t & 1 of the ring.
+    auto fetch = [&](int t) {
+        uint64_t base = batch_start_of(stream, t / CPB, nnz) + (uint64_t)((t % CPB) * kBChunk);
+        while (base >= nnz) base -= nnz;  // start < nnz: wraps more than once only when nnz < 128
+        uint32_t *dst = rec + (t & 1) * CW + lane;
+        if (base + kBChunk <= nnz) {
+            const uint32_t *src = Rw + base * 3 + lane;
 #pragma unroll
-        for (int i = 0; i < WPL; ++i) {
-            const int w = lane + i * G;
-            uint64_t rec = base + (uint64_t)(w / 3);
-            while (rec >= nnz) rec -= nnz;
-            bcp_async4(&s_rec[buf][w % 3][w / 3], Rw + rec * 3 + (w % 3));
+            for (int i = 0; i < WPL; ++i) bcp_async4(dst + i * G, src + i * G);
+        } else {
+            for (int i = 0; i < WPL; ++i) {
+                const int word = lane + i * G;
+                uint64_t r = base + (uint64_t)(word / 3);
+                while (r >= nnz) r -= nnz;
+                bcp_async4(dst + i * G, Rw + r * 3 + (word % 3));
+            }
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
-    auto load = [&](V (&dst)[NVEC], V *base, uint32_t row, bool ok) {
+    // Bit j (even): records j and j + 1 of chunk t have to go one after the other.
+    auto scan = [&](int t) {
+        uint32_t slow = 0;
 #pragma unroll
-        for (int i = 0; i < NVEC; ++i) dst[i] = ok ? __ldcg(base + (uint64_t)row * ROWV + i) : V{};
+        for (int i = 0; i < kBChunk / G; ++i) {
+            const int j = lane + i * G;
+            const uint32_t *w = rec + (t & 1) * CW + 3 * j, *w2 = rec + (t & 1) * CW + 3 * (j ^ 1);
+            const uint32_t u = w[0], v = w[1], u2 = w2[0], v2 = w2[1];
+            const bool s = (u > m1) | (v > n1) | (u2 > m1) | (v2 > n1) | (u == u2) | (v == v2);
+            slow |= ((__ballot_sync(gmask, s) >> shift) & group) << (i * G);
+        }
+        return slow;
     };
-    fetch(0, 0);
+    __syncwarp(gmask);  // the last epoch's or task's records are no longer read
+    fetch(0);
     asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncwarp(gmask);
-    uint32_t u = s_rec[0][0][0], v = s_rec[0][1][0];
-    bool ok = (u < pr.m) & (v < pr.n);
-    V fp[NVEC], fq[NVEC];
-    load(fp, P, u, ok);
-    load(fq, Q, v, ok);
+    uint32_t slow = scan(0);
+    uint32_t nu = rec[3 * half], nv = rec[3 * half + 1];  // ids of this half's next record
     for (int t = 0; t < chunks; ++t) {
-        const int buf = t & 1;
-        const bool has_next = t + 1 < chunks;
-        if (has_next) fetch(t + 1, buf ^ 1);
+        __syncwarp(gmask);  // the half refilled next is no longer read
+        if (t + 1 < chunks) fetch(t + 1);
+        const uint32_t *cur = rec + (t & 1) * CW + 3 * half;
+        const int next_half = (t & 1) ? -2 * CW : 0;  // added to an index past this chunk's end
 #pragma unroll 1
-        for (int j = 0; j < kBChunk; ++j) {
-            uint32_t un = 0xffffffffu, vn = 0xffffffffu;
-            if (j + 1 < kBChunk) {
-                un = s_rec[buf][0][j + 1];
-                vn = s_rec[buf][1][j + 1];
-            } else if (has_next) {
-                asm volatile("cp.async.wait_all;\n" ::: "memory");
-                __syncwarp(gmask);
-                un = s_rec[buf ^ 1][0][0];
-                vn = s_rec[buf ^ 1][1][0];
-            }
-            const bool okn = (un < pr.m) & (vn < pr.n);
-            V np[NVEC], nq[NVEC];
-            load(np, P, un, okn);
-            load(nq, Q, vn, okn);
-            if (ok) {
-                const float r = __uint_as_float(s_rec[buf][2][j]);
-                float s = 0.f;
-#pragma unroll
-                for (int i = 0; i < NVEC; ++i)
-#pragma unroll
-                    for (int w = 0; w < WPV; ++w) {
-                        const float2 pp = __half22float2(*reinterpret_cast<__half2 *>(&word(fp[i], w)));
-                        const float2 qq = __half22float2(*reinterpret_cast<__half2 *>(&word(fq[i], w)));
-                        s = __fmaf_rn(pp.x, qq.x, s);
-                        s = __fmaf_rn(pp.y, qq.y, s);
-                    }
-#pragma unroll
-                for (int o = G / 2; o >= 1; o >>= 1) s += __shfl_xor_sync(gmask, s, o);
-                const float err = r - s;
-                V wp[NVEC], wq[NVEC];
-#pragma unroll
-                for (int i = 0; i < NVEC; ++i)
-#pragma unroll
-                    for (int w = 0; w < WPV; ++w) {
-                        const float2 pp = __half22float2(*reinterpret_cast<__half2 *>(&word(fp[i], w)));
-                        const float2 qq = __half22float2(*reinterpret_cast<__half2 *>(&word(fq[i], w)));
-                        const float px = __fmaf_rn(lr, __fmaf_rn(err, qq.x, -__fmul_rn(pr.lp, pp.x)), pp.x);
-                        const float py = __fmaf_rn(lr, __fmaf_rn(err, qq.y, -__fmul_rn(pr.lp, pp.y)), pp.y);
-                        const float qx = __fmaf_rn(lr, __fmaf_rn(err, pp.x, -__fmul_rn(pr.lq, qq.x)), qq.x);
-                        const float qy = __fmaf_rn(lr, __fmaf_rn(err, pp.y, -__fmul_rn(pr.lq, qq.y)), qq.y);
-                        __half2 hp = __floats2half2_rn(px, py), hq = __floats2half2_rn(qx, qy);
-                        word(wp[i], w) = *reinterpret_cast<uint32_t *>(&hp);
-                        word(wq[i], w) = *reinterpret_cast<uint32_t *>(&hq);
-                    }
-#pragma unroll
-                for (int i = 0; i < NVEC; ++i) {
-                    __stcg(P + (uint64_t)u * ROWV + i, wp[i]);
-                    __stcg(Q + (uint64_t)v * ROWV + i, wq[i]);
-                }
-                if (un == u)
-#pragma unroll
-                    for (int i = 0; i < NVEC; ++i) np[i] = wp[i];
-                if (vn == v)
-#pragma unroll
-                    for (int i = 0; i < NVEC; ++i) nq[i] = wq[i];
+        for (int j = 0; j < kBChunk; j += 2, slow >>= 2) {
+            const uint32_t u = nu, v = nv;
+            if (j == kBChunk - 2) asm volatile("cp.async.wait_all;\n" ::: "memory");  // the look-ahead enters the next chunk
+            __syncwarp(gmask);  // the last pair's stores, and the next chunk's records
+            // (Past the last chunk this reads old records' ids, which are not used.)
+            const uint32_t *ahead = cur + 3 * (j + 2) + (j + 2 >= kBChunk ? next_half : 0);
+            nu = ahead[0];
+            nv = ahead[1];
+            const float r = __uint_as_float(cur[3 * j + 2]);
+            if (__builtin_expect((slow & 1u) == 0, 1)) {
+                pair_record<G, SB>(c, gmask, u, v, r);
             } else {
-                *bad = 1;
+                const bool ok = (u <= m1) & (v <= n1);
+                if (!ok) *bad = 1;
+                for (int e = 0; e < 2; ++e) {
+                    if (half == e && ok) pair_record<G, SB>(c, ((1u << H) - 1u) << (shift + e * H), u, v, r);
+                    __syncwarp(gmask);
+                }
             }
-#pragma unroll
-            for (int i = 0; i < NVEC; ++i) {
-                fp[i] = np[i];
-                fq[i] = nq[i];
-            }
-            u = un;
-            v = vn;
-            ok = okn;
         }
-        __syncwarp(gmask);
+        slow = scan(t + 1);  // (past the last chunk: old records, not used)
     }
 }
 
@@ -217,7 +270,7 @@ __global__ void __launch_bounds__(kBT, 4)
 batch_kernel(const BatchProblemDev *probs, const BatchTask *tasks, int tasks_per_epoch, int first_epoch, int n_epochs,
              int *counter, int *status) {
     constexpr int GPB = kBT / G;
-    __shared__ uint32_t s_rec[GPB][2][3][kBChunk + 1];
+    __shared__ uint32_t s_rec[GPB][2 * kBChunk * 3 + 1];  // two chunks per group, records as in memory
     const int lane = threadIdx.x % G;
     const int gib = threadIdx.x / G;
     const unsigned gmask = (G == 32) ? 0xffffffffu : (((1u << G) - 1u) << ((threadIdx.x & 31) & ~(G - 1)));
@@ -232,13 +285,13 @@ batch_kernel(const BatchProblemDev *probs, const BatchTask *tasks, int tasks_per
         const BatchProblemDev pr = probs[t.problem];
         if (pr.nnz == 0 || pr.batches == 0) continue;
         for (int ep = first_epoch; ep < first_epoch + n_epochs; ++ep) {
-            if (pr.k == 128 && G == 8) run_task<G, 16>(pr, t.worker, ep, lane, gmask, s_rec[gib], &bad);
+            if (pr.k == 128 && G == 8) run_task<G, 32>(pr, t.worker, ep, lane, gmask, s_rec[gib], &bad);
             else if ((pr.k == 128 && G == 16) || (pr.k == 64 && G == 8))
-                run_task<G, 8>(pr, t.worker, ep, lane, gmask, s_rec[gib], &bad);
+                run_task<G, 16>(pr, t.worker, ep, lane, gmask, s_rec[gib], &bad);
             else if ((pr.k == 128 && G == 32) || (pr.k == 64 && G == 16) || (pr.k == 32 && G == 8))
-                run_task<G, 4>(pr, t.worker, ep, lane, gmask, s_rec[gib], &bad);
+                run_task<G, 8>(pr, t.worker, ep, lane, gmask, s_rec[gib], &bad);
             else if ((pr.k == 64 && G == 32) || (pr.k == 32 && G == 16))
-                run_task<G, 2>(pr, t.worker, ep, lane, gmask, s_rec[gib], &bad);
+                run_task<G, 4>(pr, t.worker, ep, lane, gmask, s_rec[gib], &bad);
             else
                 bad = 1;
         }
