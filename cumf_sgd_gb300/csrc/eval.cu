@@ -16,11 +16,11 @@
 //   2. one thread per row replays the swaps on column ids (the "positive block"; with no
 //      repeated column it is the positive columns themselves);
 //   3. the block's predictions are computed (sequential fp32 FMA over k, as
-//      std::inner_product contracted to FMA) and sorted per row (CUB segmented sort);
+//      std::inner_product contracted to FMA) and sorted by (row, prediction) (CUB radix sort);
 //   4. a sweep CTA takes 16 rows: each thread predicts its columns for all 16 rows from the
 //      transposed column factors (one global load feeds 16 FMAs) and counts, by binary search
 //      in the sorted block predictions, the positives predicted higher;
-//   5. the pairs inside the block are subtracted, and per-row terms are summed in row order.
+//   5. the pairs inside the block are subtracted, and per-row terms are summed in a fixed order.
 #include <cub/cub.cuh>
 #include <thrust/iterator/counting_iterator.h>
 #include <thrust/iterator/transform_iterator.h>
@@ -93,12 +93,13 @@ __global__ void __launch_bounds__(kT) pointwise_kernel(const cumf_node *__restri
     if (threadIdx.x == 0) part[blockIdx.x] = t;
 }
 
-__global__ void ordered_sum_kernel(const double *part, int64_t count, double *out) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double s = 0;
-        for (int64_t i = 0; i < count; ++i) s += part[i];
-        *out = s;
-    }
+// Sum of `count` partials in a fixed order: thread t adds part[t], part[t + kT], ..., then
+// block_sum's tree.  (One thread adding 1,024 partials took 90 us of dependent loads.)
+__global__ void __launch_bounds__(kT) ordered_sum_kernel(const double *part, int64_t count, double *out) {
+    double s = 0;
+    for (int64_t i = threadIdx.x; i < count; i += kT) s += part[i];
+    const double t = block_sum(s);
+    if (threadIdx.x == 0) *out = t;
 }
 
 // ---- ranking criteria ---------------------------------------------------------------------
@@ -168,13 +169,31 @@ __device__ __forceinline__ float seq_predict(const float *__restrict__ P, int32_
     return isnan(z) ? b : z;
 }
 
-// Predictions of the block columns; row-major "row factors" R_f (rows x k) and "column
-// factors" C_f (cols x k) already swapped for the column-wise criteria.
-__global__ void block_pred_kernel(const uint64_t *__restrict__ pkeys, const int32_t *__restrict__ blk, int64_t total,
-                                  const float *__restrict__ Rf, int32_t rf_rows, const float *__restrict__ Cf,
-                                  int32_t cf_rows, int k, float b, float *pred) {
+// Floats as unsigned integers of the same order, and back.
+__device__ __forceinline__ uint32_t float_key(float x) {
+    const uint32_t b = __float_as_uint(x);
+    return b ^ ((b >> 31) ? 0xffffffffu : 0x80000000u);
+}
+__device__ __forceinline__ float key_float(uint32_t k) {
+    return __uint_as_float(k ^ ((k >> 31) ? 0x80000000u : 0xffffffffu));
+}
+
+// Sort keys (segment << 32 | prediction) of the block columns; row-major "row factors" R_f (rows
+// x k) and "column factors" C_f (cols x k) already swapped for the column-wise criteria.
+// seg_end[j]: segments that start at or before j.
+__global__ void block_pred_kernel(const uint64_t *__restrict__ pkeys, const int32_t *__restrict__ blk,
+                                  const int64_t *__restrict__ seg_end, int64_t total, const float *__restrict__ Rf,
+                                  int32_t rf_rows, const float *__restrict__ Cf, int32_t cf_rows, int k, float b,
+                                  uint64_t *key) {
+    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < total; j += (int64_t)gridDim.x * blockDim.x) {
+        const float z = seq_predict(Rf, rf_rows, Cf, cf_rows, k, b, key_row(pkeys[j]), blk[j]);
+        key[j] = ((uint64_t)(seg_end[j + 1] - 1) << 32) | float_key(z);
+    }
+}
+
+__global__ void unkey_kernel(const uint64_t *__restrict__ key, int64_t total, float *pred) {
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < total; j += (int64_t)gridDim.x * blockDim.x)
-        pred[j] = seq_predict(Rf, rf_rows, Cf, cf_rows, k, b, key_row(pkeys[j]), blk[j]);
+        pred[j] = key_float((uint32_t)key[j]);
 }
 
 // Number of entries of the ascending array s[0..len) greater than x.
@@ -190,8 +209,25 @@ __device__ __forceinline__ int64_t count_greater(const float *s, int64_t len, fl
     return len - lo;
 }
 
-// CTA over up to 16 active segments; threads stride over all columns [0, ncols_eff).
-// CfT is the column factors transposed (k x cf_rows).
+// CTA over up to 16 active segments; a thread predicts kSweepCols columns at a time, striding over
+// all columns [0, ncols_eff).  CfT is the column factors transposed (k x cf_rows).
+// Bound by the fp32 FMAs (rows x columns x k, in the order of mf_predict) once the operands come
+// cheaply: the 16 row factors of one k lie side by side in shared memory (four 16-byte broadcasts
+// feed 16 x kSweepCols FMAs), two rows per fma.rn.f32x2.  The rows' sorted predictions are
+// searched in shared memory where they fit (pred_cap floats for the 16 rows), without branches:
+// a row's length is the same for all threads.  10,000 x 2,000, k = 128, 70,000 positives:
+// 445 -> 215 us (one column per thread, one 4-byte broadcast per FMA, searches in L1 before).
+constexpr int kSweepCols = 2;
+constexpr int kSweepPreds = 1024;
+
+// Entries of the ascending array s[0..len) greater than x.
+__device__ __forceinline__ int count_greater_smem(const float *s, int len, float x) {
+    int lo = 0;  // entries known to be <= x
+    for (int step = len > 0 ? 1 << (31 - __clz(len)) : 0; step > 0; step >>= 1)
+        if (lo + step <= len && !(s[lo + step - 1] > x)) lo += step;
+    return len - lo;
+}
+
 __global__ void __launch_bounds__(kT) sweep_kernel(const int64_t *__restrict__ active, int64_t nactive,
                                                    const int64_t *__restrict__ seg_off,
                                                    const int32_t *__restrict__ seg_row,
@@ -199,10 +235,11 @@ __global__ void __launch_bounds__(kT) sweep_kernel(const int64_t *__restrict__ a
                                                    const float *__restrict__ Rf, int32_t rf_rows,
                                                    const float *__restrict__ CfT, int32_t cf_rows,
                                                    int32_t ncols_eff, int k, float b,
-                                                   unsigned long long *seg_count) {
-    extern __shared__ float s_p[];  // kRowsPerSweep x k row factors
+                                                   int pred_cap, unsigned long long *seg_count) {
+    extern __shared__ __align__(16) float s_p[];  // k x kRowsPerSweep row factors, then pred_cap predictions
+    float *const s_pred = s_p + kRowsPerSweep * k;
     __shared__ int64_t s_seg[kRowsPerSweep], s_off[kRowsPerSweep], s_len[kRowsPerSweep];
-    __shared__ int s_valid[kRowsPerSweep];
+    __shared__ int s_valid[kRowsPerSweep], s_at[kRowsPerSweep + 1];
     __shared__ unsigned long long s_cnt[kRowsPerSweep];
     const int64_t g0 = (int64_t)blockIdx.x * kRowsPerSweep;
     const int nr = (nactive - g0 < kRowsPerSweep) ? (int)(nactive - g0) : kRowsPerSweep;
@@ -223,31 +260,71 @@ __global__ void __launch_bounds__(kT) sweep_kernel(const int64_t *__restrict__ a
         }
     }
     __syncthreads();
+    if (threadIdx.x == 0) {
+        int64_t at = 0;
+        for (int r = 0; r < kRowsPerSweep; ++r) {
+            s_at[r] = (int)min(at, (int64_t)pred_cap + 1);
+            at += s_len[r];
+        }
+        s_at[kRowsPerSweep] = (int)min(at, (int64_t)pred_cap + 1);
+    }
     for (int idx = threadIdx.x; idx < kRowsPerSweep * k; idx += blockDim.x) {
         const int r = idx / k, t = idx % k;
-        s_p[idx] = (r < nr && s_valid[r]) ? Rf[(int64_t)seg_row[s_seg[r]] * k + t] : 0.f;
+        s_p[t * kRowsPerSweep + r] = (r < nr && s_valid[r]) ? Rf[(int64_t)seg_row[s_seg[r]] * k + t] : 0.f;
+    }
+    __syncthreads();
+    const bool in_smem = s_at[kRowsPerSweep] <= pred_cap;
+    if (in_smem) {
+        for (int r = threadIdx.x / 16; r < nr; r += kT / 16)
+            for (int i = threadIdx.x % 16; i < (int)s_len[r]; i += 16) s_pred[s_at[r] + i] = sorted_pred[s_off[r] + i];
     }
     __syncthreads();
     unsigned long long cnt[kRowsPerSweep];
 #pragma unroll
     for (int r = 0; r < kRowsPerSweep; ++r) cnt[r] = 0;
-    for (int32_t j = threadIdx.x; j < ncols_eff; j += blockDim.x) {
-        float acc[kRowsPerSweep];
+    for (int32_t j0 = threadIdx.x; j0 < ncols_eff; j0 += kSweepCols * kT) {
+        float2 acc[kSweepCols][kRowsPerSweep / 2];
 #pragma unroll
-        for (int r = 0; r < kRowsPerSweep; ++r) acc[r] = 0.f;
-        const bool in_model = j < cf_rows;
-        if (in_model) {
+        for (int c = 0; c < kSweepCols; ++c)
+#pragma unroll
+            for (int r = 0; r < kRowsPerSweep / 2; ++r) acc[c][r] = make_float2(0.f, 0.f);
+        // Columns past the model read column cf_rows - 1 and are not counted with it.
+        const float *q[kSweepCols];
+        bool in_model[kSweepCols];
+#pragma unroll
+        for (int c = 0; c < kSweepCols; ++c) {
+            in_model[c] = j0 + c * kT < cf_rows;
+            q[c] = CfT + (in_model[c] ? j0 + c * kT : cf_rows - 1);
+        }
+        if (cf_rows > 0) {
+#pragma unroll 4
             for (int t = 0; t < k; ++t) {
-                const float q = __ldg(CfT + (int64_t)t * cf_rows + j);
+                float2 p[kRowsPerSweep / 2];
 #pragma unroll
-                for (int r = 0; r < kRowsPerSweep; ++r) acc[r] = __fmaf_rn(s_p[r * k + t], q, acc[r]);
+                for (int r = 0; r < kRowsPerSweep / 4; ++r) {
+                    const float4 x = reinterpret_cast<const float4 *>(s_p)[t * (kRowsPerSweep / 4) + r];
+                    p[2 * r] = make_float2(x.x, x.y);
+                    p[2 * r + 1] = make_float2(x.z, x.w);
+                }
+#pragma unroll
+                for (int c = 0; c < kSweepCols; ++c) {
+                    const float x = __ldg(q[c] + (int64_t)t * cf_rows);
+#pragma unroll
+                    for (int r = 0; r < kRowsPerSweep / 2; ++r) acc[c][r] = __ffma2_rn(p[r], make_float2(x, x), acc[c][r]);
+                }
             }
         }
 #pragma unroll
-        for (int r = 0; r < kRowsPerSweep; ++r) {
-            if (r >= nr) continue;
-            const float z = (in_model && s_valid[r] && !isnan(acc[r])) ? acc[r] : b;
-            cnt[r] += (unsigned long long)count_greater(sorted_pred + s_off[r], s_len[r], z);
+        for (int c = 0; c < kSweepCols; ++c) {
+            if (j0 + c * kT >= ncols_eff) continue;
+#pragma unroll
+            for (int r = 0; r < kRowsPerSweep; ++r) {
+                if (r >= nr) continue;
+                const float d = (r & 1) ? acc[c][r / 2].y : acc[c][r / 2].x;
+                const float z = (in_model[c] && s_valid[r] && !isnan(d)) ? d : b;
+                cnt[r] += (unsigned long long)(in_smem ? count_greater_smem(s_pred + s_at[r], (int)s_len[r], z)
+                                                       : count_greater(sorted_pred + s_off[r], s_len[r], z));
+            }
         }
     }
 #pragma unroll
@@ -283,20 +360,39 @@ __global__ void row_terms_kernel(const int64_t *__restrict__ seg_off, int64_t ns
     pos_out[s] = pos;
 }
 
-// Row-order sums (the reference's serial order) of the per-row terms.
-__global__ void finish_kernel(const double *mpr, const double *auc, const int64_t *pos, int64_t nseg, double *out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// Sums of the per-row terms in a fixed order, one block: thread t adds rows t, t + kFinishT, ...,
+// then a tree (one thread adding 10,000 rows in turn took 1.4 ms).
+constexpr int kFinishT = 1024;
+__global__ void __launch_bounds__(kFinishT) finish_kernel(const double *mpr, const double *auc, const int64_t *pos,
+                                                          int64_t nseg, double *out) {
+    __shared__ double s_m[kFinishT], s_a[kFinishT];
+    __shared__ unsigned long long s_n[kFinishT], s_p[kFinishT];
     double sm = 0, sa = 0;
-    long long tm = 0, tp = 0;
-    for (int64_t s = 0; s < nseg; ++s) {
+    unsigned long long tm = 0, tp = 0;
+    for (int64_t s = threadIdx.x; s < nseg; s += kFinishT) {
         if (pos[s] == 0) continue;
         sm += mpr[s];
         sa += auc[s];
         tm += 1;
-        tp += pos[s];
+        tp += (unsigned long long)pos[s];
     }
-    out[0] = sm / (double)tp;
-    out[1] = sa / (double)tm;
+    s_m[threadIdx.x] = sm;
+    s_a[threadIdx.x] = sa;
+    s_n[threadIdx.x] = tm;
+    s_p[threadIdx.x] = tp;
+    for (int w = kFinishT / 2; w >= 1; w >>= 1) {
+        __syncthreads();
+        if ((int)threadIdx.x < w) {
+            s_m[threadIdx.x] += s_m[threadIdx.x + w];
+            s_a[threadIdx.x] += s_a[threadIdx.x + w];
+            s_n[threadIdx.x] += s_n[threadIdx.x + w];
+            s_p[threadIdx.x] += s_p[threadIdx.x + w];
+        }
+    }
+    if (threadIdx.x == 0) {
+        out[0] = s_m[0] / (double)s_p[0];
+        out[1] = s_a[0] / (double)s_n[0];
+    }
 }
 
 __global__ void transpose_f32_kernel(const float *__restrict__ in, int64_t rows, int k, float *out) {
@@ -420,23 +516,26 @@ int mpr_auc_device(const cumf_node *d_R, int64_t nnz, int32_t prob_m, int32_t pr
                                                    seg_off.as<int64_t>(), seg_row.as<int32_t>());
     CUMF_CUDA(cudaMemcpyAsync(seg_off.as<int64_t>() + nseg, &total, sizeof(int64_t), cudaMemcpyHostToDevice, s));
     // 3. positive blocks, their predictions, sorted per row.
-    DevBuf blk, pred, spred;
+    // One radix sort of (segment, prediction) over all positives: a segmented sort launches a
+    // block per row, 0.93 ms for 10,000 rows of about 7, against 0.08 for this.
+    DevBuf blk, pkey, spkey, spred;
     CUMF_CUDA(blk.alloc(total * 4));
-    CUMF_CUDA(pred.alloc(total * 4));
+    CUMF_CUDA(pkey.alloc(total * 8));
+    CUMF_CUDA(spkey.alloc(total * 8));
     CUMF_CUDA(spred.alloc(total * 4));
     block_kernel<<<grid_of(nseg), kT, 0, s>>>(pkeys.as<uint64_t>(), seg_off.as<int64_t>(), nseg, blk.as<int32_t>());
-    block_pred_kernel<<<grid_of(total), kT, 0, s>>>(pkeys.as<uint64_t>(), blk.as<int32_t>(), total, Rf, rf_rows, Cf,
-                                                    cf_rows, k, b, pred.as<float>());
+    block_pred_kernel<<<grid_of(total), kT, 0, s>>>(pkeys.as<uint64_t>(), blk.as<int32_t>(), heads.as<int64_t>(), total, Rf,
+                                                    rf_rows, Cf, cf_rows, k, b, pkey.as<uint64_t>());
     CUMF_CUDA(cudaGetLastError());
     {
+        int end_bit = 33;
+        while (end_bit < 64 && ((nseg - 1) >> (end_bit - 32)) != 0) ++end_bit;
         size_t tb4 = 0;
-        CUMF_CUDA(cub::DeviceSegmentedRadixSort::SortKeys(nullptr, tb4, pred.as<float>(), spred.as<float>(), total,
-                                                          nseg, seg_off.as<int64_t>(), seg_off.as<int64_t>() + 1, 0,
-                                                          32, s));
+        CUMF_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, tb4, pkey.as<uint64_t>(), spkey.as<uint64_t>(), total, 0, end_bit, s));
         CUMF_CUDA(tmp.alloc(std::max<size_t>(tb4, 16)));
-        CUMF_CUDA(cub::DeviceSegmentedRadixSort::SortKeys(tmp.p, tb4, pred.as<float>(), spred.as<float>(), total,
-                                                          nseg, seg_off.as<int64_t>(), seg_off.as<int64_t>() + 1, 0,
-                                                          32, s));
+        CUMF_CUDA(cub::DeviceRadixSort::SortKeys(tmp.p, tb4, pkey.as<uint64_t>(), spkey.as<uint64_t>(), total, 0, end_bit, s));
+        unkey_kernel<<<grid_of(total), kT, 0, s>>>(spkey.as<uint64_t>(), total, spred.as<float>());
+        CUMF_CUDA(cudaGetLastError());
     }
     // 4. active rows and the column sweep.
     DevBuf aflag, active, nact;
@@ -464,14 +563,16 @@ int mpr_auc_device(const cumf_node *d_R, int64_t nnz, int32_t prob_m, int32_t pr
             dim3 tg((unsigned)((cf_rows + 31) / 32), (unsigned)((k + 31) / 32));
             transpose_f32_kernel<<<tg, dim3(32, 8), 0, s>>>(Cf, cf_rows, k, cfT.as<float>());
         }
-        const size_t smem = (size_t)kRowsPerSweep * k * sizeof(float);
-        if (smem > 48 * 1024)
+        const size_t factors = (size_t)kRowsPerSweep * k * sizeof(float);
+        const int pred_cap = factors <= 200 * 1024 ? kSweepPreds : 0;  // (long rows of factors leave no room)
+        const size_t smem = factors + pred_cap * sizeof(float);
+        if (smem > 46 * 1024)  // with the static arrays, more than the default 48 KB
             CUMF_CUDA(cudaFuncSetAttribute(sweep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         const int64_t groups = (nactive + kRowsPerSweep - 1) / kRowsPerSweep;
         if (groups > 0x7fffffffll) return fail(CUMF_ERR_ARG, "evaluate: too many rows");
         sweep_kernel<<<(unsigned)groups, kT, smem, s>>>(active.as<int64_t>(), nactive, seg_off.as<int64_t>(),
                                                         seg_row.as<int32_t>(), spred.as<float>(), Rf, rf_rows,
-                                                        cfT.as<float>(), cf_rows, cols, k, b,
+                                                        cfT.as<float>(), cf_rows, cols, k, b, pred_cap,
                                                         segcnt.as<unsigned long long>());
         CUMF_CUDA(cudaGetLastError());
     }
@@ -483,7 +584,7 @@ int mpr_auc_device(const cumf_node *d_R, int64_t nnz, int32_t prob_m, int32_t pr
     row_terms_kernel<<<grid_of(nseg), kT, 0, s>>>(seg_off.as<int64_t>(), nseg, spred.as<float>(),
                                                   segcnt.as<unsigned long long>(), cols, mpr.as<double>(),
                                                   auc.as<double>(), posb.as<int64_t>());
-    finish_kernel<<<1, 32, 0, s>>>(mpr.as<double>(), auc.as<double>(), posb.as<int64_t>(), nseg, res.as<double>());
+    finish_kernel<<<1, kFinishT, 0, s>>>(mpr.as<double>(), auc.as<double>(), posb.as<int64_t>(), nseg, res.as<double>());
     CUMF_CUDA(cudaGetLastError());
     CUMF_CUDA(cudaMemcpyAsync(out, res.p, 16, cudaMemcpyDeviceToHost, s));
     CUMF_CUDA(cudaStreamSynchronize(s));
@@ -547,7 +648,7 @@ extern "C" int cumf_evaluate(const cumf_problem *te, const cumf_model *model, in
         case kLOGLOSS: pointwise_kernel<kLOGLOSS><<<kBlocks, kT, 0, stream.s>>>(R, nnz, P, m, Q, n, model->k, model->b, d_part.as<double>()); break;
         default: pointwise_kernel<kACC><<<kBlocks, kT, 0, stream.s>>>(R, nnz, P, m, Q, n, model->k, model->b, d_part.as<double>()); break;
     }
-    ordered_sum_kernel<<<1, 32, 0, stream.s>>>(d_part.as<double>(), kBlocks, d_sum.as<double>());
+    ordered_sum_kernel<<<1, kT, 0, stream.s>>>(d_part.as<double>(), kBlocks, d_sum.as<double>());
     CUMF_CUDA(cudaGetLastError());
     double sum = 0;
     CUMF_CUDA(cudaMemcpyAsync(&sum, d_sum.p, sizeof(double), cudaMemcpyDeviceToHost, stream.s));
