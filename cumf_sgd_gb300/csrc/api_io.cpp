@@ -133,6 +133,7 @@ extern "C" int cumf_release_host_cache(void) {
     for (auto &blk : c.free_blocks) cudaFreeHost(blk.first);
     c.free_blocks.clear();
     c.cached_bytes = 0;
+    scratch_release();
     return CUMF_OK;
 }
 

@@ -56,12 +56,12 @@ struct EpochEval {
         m = m_;
         n = n_;
         k = k_;
-        CUMF_CUDA(d_va.alloc(std::max<int64_t>(1, v->nnz) * sizeof(cumf_node)));
+        CUMF_CUDA(d_va.alloc(std::max<int64_t>(1, v->nnz) * sizeof(cumf_node), s));
         if (v->nnz) CUMF_CUDA(cudaMemcpyAsync(d_va.p, v->R, v->nnz * sizeof(cumf_node), cudaMemcpyHostToDevice, s));
-        CUMF_CUDA(d_pf.alloc((size_t)m * k * sizeof(float)));
-        CUMF_CUDA(d_qf.alloc((size_t)n * k * sizeof(float)));
-        CUMF_CUDA(d_part.alloc(rmse_blocks(v->nnz) * sizeof(double)));
-        CUMF_CUDA(d_sum.alloc(sizeof(double)));
+        CUMF_CUDA(d_pf.alloc((size_t)m * k * sizeof(float), s));
+        CUMF_CUDA(d_qf.alloc((size_t)n * k * sizeof(float), s));
+        CUMF_CUDA(d_part.alloc(rmse_blocks(v->nnz) * sizeof(double), s));
+        CUMF_CUDA(d_sum.alloc(sizeof(double), s));
         return CUMF_OK;
     }
     // Exports the current factors exactly as the final model would be and evaluates.
@@ -204,22 +204,22 @@ int train_mode_a(const cumf_problem *tr, const cumf_problem *va, const cumf_para
     cudaStream_t s = stream.s;
 
     DevBuf d_R, d_part, d_small, d_pmap, d_qmap, d_P, d_Q, d_lr, d_status, d_pf, d_qf;
-    CUMF_CUDA(d_R.alloc(std::max<int64_t>(1, nnz) * sizeof(cumf_node)));
+    CUMF_CUDA(d_R.alloc(std::max<int64_t>(1, nnz) * sizeof(cumf_node), s));
     if (nnz) CUMF_CUDA(cudaMemcpyAsync(d_R.p, tr->R, nnz * sizeof(cumf_node), cudaMemcpyHostToDevice, s));
     const bool use_ck = ck && ck->path && ck->path[0];
     DevBuf d_dig;
     unsigned long long records_digest = 0;
     if (use_ck) {  // fingerprint of the caller's ratings, before they are permuted and scaled
-        CUMF_CUDA(d_dig.alloc(sizeof(unsigned long long)));
+        CUMF_CUDA(d_dig.alloc(sizeof(unsigned long long), s));
         CUMF_CUDA(launch_digest(d_R.p, (uint64_t)nnz * sizeof(cumf_node), d_dig.as<unsigned long long>(), s));
         CUMF_CUDA(cudaMemcpyAsync(&records_digest, d_dig.p, sizeof(records_digest), cudaMemcpyDeviceToHost, s));
     }
 
     // collect_data on the device.
     Prepared pr;
-    CUMF_CUDA(d_part.alloc(2 * stats_blocks(nnz) * sizeof(double)));
-    CUMF_CUDA(d_small.alloc(4 * sizeof(double)));
-    CUMF_CUDA(d_status.alloc(sizeof(int)));
+    CUMF_CUDA(d_part.alloc(2 * stats_blocks(nnz) * sizeof(double), s));
+    CUMF_CUDA(d_small.alloc(4 * sizeof(double), s));
+    CUMF_CUDA(d_status.alloc(sizeof(int), s));
     CUMF_CUDA(cudaMemsetAsync(d_status.p, 0, sizeof(int), s));
     CUMF_CUDA(launch_rating_stats(d_R.as<cumf_node>(), nnz, d_part.as<double>(), d_small.as<double>(), s));
     double sums[2] = {0, 0};
@@ -227,8 +227,8 @@ int train_mode_a(const cumf_problem *tr, const cumf_problem *va, const cumf_para
 
     // Id maps on the host (sequential glibc stream) while the stats run.
     make_maps((uint32_t)p.seed, m, n, pr);
-    CUMF_CUDA(d_pmap.alloc((size_t)m * sizeof(int32_t)));
-    CUMF_CUDA(d_qmap.alloc((size_t)n * sizeof(int32_t)));
+    CUMF_CUDA(d_pmap.alloc((size_t)m * sizeof(int32_t), s));
+    CUMF_CUDA(d_qmap.alloc((size_t)n * sizeof(int32_t), s));
     CUMF_CUDA(cudaMemcpyAsync(d_pmap.p, pr.pmap.data(), (size_t)m * sizeof(int32_t), cudaMemcpyHostToDevice, s));
     CUMF_CUDA(cudaMemcpyAsync(d_qmap.p, pr.qmap.data(), (size_t)n * sizeof(int32_t), cudaMemcpyHostToDevice, s));
     CUMF_CUDA(cudaStreamSynchronize(s));
@@ -266,15 +266,15 @@ int train_mode_a(const cumf_problem *tr, const cumf_problem *va, const cumf_para
 
     // init_model: every row, including rows without ratings (sgd.cu:548-591).
     const int eb = elem_bytes(p.precision);
-    CUMF_CUDA(d_P.alloc((size_t)m_rows * k * eb));
-    CUMF_CUDA(d_Q.alloc((size_t)n_rows * k * eb));
+    CUMF_CUDA(d_P.alloc((size_t)m_rows * k * eb, s));
+    CUMF_CUDA(d_Q.alloc((size_t)n_rows * k * eb, s));
     CUMF_CUDA(launch_init_factors(d_P.p, m, k, p.precision, p.seed, 1, s));
     CUMF_CUDA(launch_init_factors(d_Q.p, n, k, p.precision, p.seed, 2, s));
     if (init) {  // starting factors for the first init->m users and init->n items
         const float f0 = (float)sqrt(pr.scale);
         const int64_t mi = std::min<int64_t>(init->m, m), ni = std::min<int64_t>(init->n, n);
         DevBuf tmp;
-        CUMF_CUDA(tmp.alloc((size_t)std::max(mi, ni) * k * sizeof(float)));
+        CUMF_CUDA(tmp.alloc((size_t)std::max(mi, ni) * k * sizeof(float), s));
         const bool on_device = init->pinned == 2;  // P and Q are device addresses
         if (mi > 0) {
             const float *src = init->P;
@@ -300,14 +300,14 @@ int train_mode_a(const cumf_problem *tr, const cumf_problem *va, const cumf_para
 
     std::vector<float> lr(std::max(1, p.num_iters + 4));
     cumf_lr_schedule(p.alpha, p.beta, p.lrate, (int)lr.size(), lr.data());
-    CUMF_CUDA(d_lr.alloc(lr.size() * sizeof(float)));
+    CUMF_CUDA(d_lr.alloc(lr.size() * sizeof(float), s));
     CUMF_CUDA(cudaMemcpyAsync(d_lr.p, lr.data(), lr.size() * sizeof(float), cudaMemcpyHostToDevice, s));
 
     // Deterministic schedule: the shuffled, scaled ratings stably sorted into G x G blocks.
     DevBuf d_S, d_off;
     if (strata_g > 0 && nnz > 0) {
-        CUMF_CUDA(d_S.alloc((size_t)nnz * sizeof(cumf_node)));
-        CUMF_CUDA(d_off.alloc(((size_t)strata_g * strata_g + 1) * sizeof(unsigned long long)));
+        CUMF_CUDA(d_S.alloc((size_t)nnz * sizeof(cumf_node), s));
+        CUMF_CUDA(d_off.alloc(((size_t)strata_g * strata_g + 1) * sizeof(unsigned long long), s));
         if (int rc = strata_layout(d_R.as<cumf_node>(), nnz, strata_g, d_S.as<cumf_node>(),
                                    d_off.as<unsigned long long>(), s))
             return rc;
@@ -465,8 +465,8 @@ int train_mode_a(const cumf_problem *tr, const cumf_problem *va, const cumf_para
         pf = d_R.as<float>();
         qf = pf + (size_t)m * k;
     } else {
-        CUMF_CUDA(d_pf.alloc(pfb));
-        CUMF_CUDA(d_qf.alloc(qfb));
+        CUMF_CUDA(d_pf.alloc(pfb, s));
+        CUMF_CUDA(d_qf.alloc(qfb, s));
         pf = d_pf.as<float>();
         qf = d_qf.as<float>();
     }
@@ -660,11 +660,11 @@ int cumf_rmse(const cumf_problem *te, const cumf_model *model, double *out) {
     CUMF_CUDA(cudaStreamCreateWithFlags(&stream.s, cudaStreamNonBlocking));
     DevBuf d_R, d_P, d_Q, d_part, d_sum;
     const size_t pb = (size_t)model->m * model->k * sizeof(float), qb = (size_t)model->n * model->k * sizeof(float);
-    CUMF_CUDA(d_R.alloc(te->nnz * sizeof(cumf_node)));
-    CUMF_CUDA(d_P.alloc(pb));
-    CUMF_CUDA(d_Q.alloc(qb));
-    CUMF_CUDA(d_part.alloc(rmse_blocks(te->nnz) * sizeof(double)));
-    CUMF_CUDA(d_sum.alloc(sizeof(double)));
+    CUMF_CUDA(d_R.alloc(te->nnz * sizeof(cumf_node), stream.s));
+    CUMF_CUDA(d_P.alloc(pb, stream.s));
+    CUMF_CUDA(d_Q.alloc(qb, stream.s));
+    CUMF_CUDA(d_part.alloc(rmse_blocks(te->nnz) * sizeof(double), stream.s));
+    CUMF_CUDA(d_sum.alloc(sizeof(double), stream.s));
     CUMF_CUDA(cudaMemcpyAsync(d_R.p, te->R, te->nnz * sizeof(cumf_node), cudaMemcpyHostToDevice, stream.s));
     if (pb) CUMF_CUDA(cudaMemcpyAsync(d_P.p, model->P, pb, cudaMemcpyHostToDevice, stream.s));
     if (qb) CUMF_CUDA(cudaMemcpyAsync(d_Q.p, model->Q, qb, cudaMemcpyHostToDevice, stream.s));
@@ -731,8 +731,8 @@ int cumf_dev_rating_stats(const cumf_node *d_R, int64_t nnz, double *mean, doubl
     if (nnz < 0 || (nnz > 0 && !d_R) || !mean || !std_dev) return fail(CUMF_ERR_ARG, "rating_stats: bad arguments");
     cudaStream_t s = (cudaStream_t)stream;
     DevBuf part, sum;
-    CUMF_CUDA(part.alloc(2 * stats_blocks(nnz) * sizeof(double)));
-    CUMF_CUDA(sum.alloc(2 * sizeof(double)));
+    CUMF_CUDA(part.alloc(2 * stats_blocks(nnz) * sizeof(double), s));
+    CUMF_CUDA(sum.alloc(2 * sizeof(double), s));
     CUMF_CUDA(launch_rating_stats(d_R, nnz, part.as<double>(), sum.as<double>(), s));
     double h[2];
     CUMF_CUDA(cudaMemcpyAsync(h, sum.p, sizeof(h), cudaMemcpyDeviceToHost, s));
@@ -769,8 +769,8 @@ int cumf_dev_rmse(const cumf_node *d_R, int64_t nnz, const float *d_P, int32_t m
     }
     cudaStream_t s = (cudaStream_t)stream;
     DevBuf part, sum;
-    CUMF_CUDA(part.alloc(rmse_blocks(nnz) * sizeof(double)));
-    CUMF_CUDA(sum.alloc(sizeof(double)));
+    CUMF_CUDA(part.alloc(rmse_blocks(nnz) * sizeof(double), s));
+    CUMF_CUDA(sum.alloc(sizeof(double), s));
     CUMF_CUDA(launch_rmse(d_R, nnz, d_P, m, d_Q, n, k, b, part.as<double>(), sum.as<double>(), s));
     double h = 0;
     CUMF_CUDA(cudaMemcpyAsync(&h, sum.p, sizeof(double), cudaMemcpyDeviceToHost, s));

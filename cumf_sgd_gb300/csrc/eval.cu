@@ -456,11 +456,11 @@ int mpr_auc_device(const cumf_node *d_R, int64_t nnz, int32_t prob_m, int32_t pr
     const float *Cf = transpose ? d_P : d_Q;
     const int32_t cf_rows = transpose ? pm : qn;
     DevBuf keys, vals, skeys, svals, bad, idx, pidx, npos, tmp;
-    CUMF_CUDA(keys.alloc(nnz * 8));
-    CUMF_CUDA(vals.alloc(nnz * 4));
-    CUMF_CUDA(skeys.alloc(nnz * 8));
-    CUMF_CUDA(svals.alloc(nnz * 4));
-    CUMF_CUDA(bad.alloc(sizeof(int)));
+    CUMF_CUDA(keys.alloc(nnz * 8, s));
+    CUMF_CUDA(vals.alloc(nnz * 4, s));
+    CUMF_CUDA(skeys.alloc(nnz * 8, s));
+    CUMF_CUDA(svals.alloc(nnz * 4, s));
+    CUMF_CUDA(bad.alloc(sizeof(int), s));
     CUMF_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(int), s));
     keys_kernel<<<grid_of(nnz), kT, 0, s>>>(d_R, nnz, transpose, rows, cols, keys.as<uint64_t>(), vals.as<float>(),
                                             bad.as<int>());
@@ -469,19 +469,19 @@ int mpr_auc_device(const cumf_node *d_R, int64_t nnz, int32_t prob_m, int32_t pr
     size_t tb = 0;
     CUMF_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, keys.as<uint64_t>(), skeys.as<uint64_t>(), vals.as<float>(),
                                               svals.as<float>(), nnz, 0, 64, s));
-    CUMF_CUDA(tmp.alloc(tb));
+    CUMF_CUDA(tmp.alloc(tb, s));
     CUMF_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tb, keys.as<uint64_t>(), skeys.as<uint64_t>(), vals.as<float>(),
                                               svals.as<float>(), nnz, 0, 64, s));
     DevBuf pkeys, ntot;
-    CUMF_CUDA(pkeys.alloc(nnz * 8));
-    CUMF_CUDA(ntot.alloc(sizeof(int64_t)));
+    CUMF_CUDA(pkeys.alloc(nnz * 8, s));
+    CUMF_CUDA(ntot.alloc(sizeof(int64_t), s));
     {
         auto flags = thrust::make_transform_iterator(thrust::counting_iterator<int64_t>(0),
                                                      PositiveFlag{svals.as<float>()});
         size_t tb2 = 0;
         CUMF_CUDA(cub::DeviceSelect::Flagged(nullptr, tb2, skeys.as<uint64_t>(), flags, pkeys.as<uint64_t>(),
                                              ntot.as<int64_t>(), nnz, s));
-        CUMF_CUDA(tmp.alloc(std::max(tb, tb2)));
+        CUMF_CUDA(tmp.alloc(std::max(tb, tb2), s));
         CUMF_CUDA(cub::DeviceSelect::Flagged(tmp.p, tb2, skeys.as<uint64_t>(), flags, pkeys.as<uint64_t>(),
                                              ntot.as<int64_t>(), nnz, s));
     }
@@ -497,21 +497,21 @@ int mpr_auc_device(const cumf_node *d_R, int64_t nnz, int32_t prob_m, int32_t pr
     }
     // 2. row segments of the positives.
     DevBuf heads, seg_off, seg_row, nseg_d;
-    CUMF_CUDA(heads.alloc((total + 1) * 8));
+    CUMF_CUDA(heads.alloc((total + 1) * 8, s));
     {
         auto flags = thrust::make_transform_iterator(thrust::counting_iterator<int64_t>(0),
                                                      HeadFlag{pkeys.as<uint64_t>(), total});
         size_t tb3 = 0;
         CUMF_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb3, flags, heads.as<int64_t>(), total + 1, s));
-        CUMF_CUDA(tmp.alloc(std::max<size_t>(tb3, 16)));
+        CUMF_CUDA(tmp.alloc(std::max<size_t>(tb3, 16), s));
         CUMF_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, tb3, flags, heads.as<int64_t>(), total + 1, s));
     }
     // heads[total] = number of segments.
     int64_t nseg = 0;
     CUMF_CUDA(cudaMemcpyAsync(&nseg, heads.as<int64_t>() + total, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     CUMF_CUDA(cudaStreamSynchronize(s));
-    CUMF_CUDA(seg_off.alloc((nseg + 1) * 8));
-    CUMF_CUDA(seg_row.alloc(nseg * 4 + 4));
+    CUMF_CUDA(seg_off.alloc((nseg + 1) * 8, s));
+    CUMF_CUDA(seg_row.alloc(nseg * 4 + 4, s));
     seg_heads_kernel<<<grid_of(total), kT, 0, s>>>(pkeys.as<uint64_t>(), total, heads.as<int64_t>(),
                                                    seg_off.as<int64_t>(), seg_row.as<int32_t>());
     CUMF_CUDA(cudaMemcpyAsync(seg_off.as<int64_t>() + nseg, &total, sizeof(int64_t), cudaMemcpyHostToDevice, s));
@@ -519,10 +519,10 @@ int mpr_auc_device(const cumf_node *d_R, int64_t nnz, int32_t prob_m, int32_t pr
     // One radix sort of (segment, prediction) over all positives: a segmented sort launches a
     // block per row, 0.93 ms for 10,000 rows of about 7, against 0.08 for this.
     DevBuf blk, pkey, spkey, spred;
-    CUMF_CUDA(blk.alloc(total * 4));
-    CUMF_CUDA(pkey.alloc(total * 8));
-    CUMF_CUDA(spkey.alloc(total * 8));
-    CUMF_CUDA(spred.alloc(total * 4));
+    CUMF_CUDA(blk.alloc(total * 4, s));
+    CUMF_CUDA(pkey.alloc(total * 8, s));
+    CUMF_CUDA(spkey.alloc(total * 8, s));
+    CUMF_CUDA(spred.alloc(total * 4, s));
     block_kernel<<<grid_of(nseg), kT, 0, s>>>(pkeys.as<uint64_t>(), seg_off.as<int64_t>(), nseg, blk.as<int32_t>());
     block_pred_kernel<<<grid_of(total), kT, 0, s>>>(pkeys.as<uint64_t>(), blk.as<int32_t>(), heads.as<int64_t>(), total, Rf,
                                                     rf_rows, Cf, cf_rows, k, b, pkey.as<uint64_t>());
@@ -532,22 +532,22 @@ int mpr_auc_device(const cumf_node *d_R, int64_t nnz, int32_t prob_m, int32_t pr
         while (end_bit < 64 && ((nseg - 1) >> (end_bit - 32)) != 0) ++end_bit;
         size_t tb4 = 0;
         CUMF_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, tb4, pkey.as<uint64_t>(), spkey.as<uint64_t>(), total, 0, end_bit, s));
-        CUMF_CUDA(tmp.alloc(std::max<size_t>(tb4, 16)));
+        CUMF_CUDA(tmp.alloc(std::max<size_t>(tb4, 16), s));
         CUMF_CUDA(cub::DeviceRadixSort::SortKeys(tmp.p, tb4, pkey.as<uint64_t>(), spkey.as<uint64_t>(), total, 0, end_bit, s));
         unkey_kernel<<<grid_of(total), kT, 0, s>>>(spkey.as<uint64_t>(), total, spred.as<float>());
         CUMF_CUDA(cudaGetLastError());
     }
     // 4. active rows and the column sweep.
     DevBuf aflag, active, nact;
-    CUMF_CUDA(aflag.alloc(nseg * 8));
-    CUMF_CUDA(active.alloc(nseg * 8));
-    CUMF_CUDA(nact.alloc(8));
+    CUMF_CUDA(aflag.alloc(nseg * 8, s));
+    CUMF_CUDA(active.alloc(nseg * 8, s));
+    CUMF_CUDA(nact.alloc(8, s));
     active_kernel<<<grid_of(nseg), kT, 0, s>>>(seg_off.as<int64_t>(), nseg, cols, aflag.as<int64_t>());
     {
         size_t tb5 = 0;
         CUMF_CUDA(cub::DeviceSelect::Flagged(nullptr, tb5, thrust::counting_iterator<int64_t>(0), aflag.as<int64_t>(),
                                              active.as<int64_t>(), nact.as<int64_t>(), nseg, s));
-        CUMF_CUDA(tmp.alloc(std::max<size_t>(tb5, 16)));
+        CUMF_CUDA(tmp.alloc(std::max<size_t>(tb5, 16), s));
         CUMF_CUDA(cub::DeviceSelect::Flagged(tmp.p, tb5, thrust::counting_iterator<int64_t>(0), aflag.as<int64_t>(),
                                              active.as<int64_t>(), nact.as<int64_t>(), nseg, s));
     }
@@ -555,10 +555,10 @@ int mpr_auc_device(const cumf_node *d_R, int64_t nnz, int32_t prob_m, int32_t pr
     CUMF_CUDA(cudaMemcpyAsync(&nactive, nact.p, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     CUMF_CUDA(cudaStreamSynchronize(s));
     DevBuf cfT, segcnt, mpr, auc, posb, res;
-    CUMF_CUDA(segcnt.alloc(nseg * 8));
+    CUMF_CUDA(segcnt.alloc(nseg * 8, s));
     CUMF_CUDA(cudaMemsetAsync(segcnt.p, 0, nseg * 8, s));
     if (nactive > 0) {
-        CUMF_CUDA(cfT.alloc((size_t)cf_rows * k * 4));
+        CUMF_CUDA(cfT.alloc((size_t)cf_rows * k * 4, s));
         if (cf_rows > 0) {
             dim3 tg((unsigned)((cf_rows + 31) / 32), (unsigned)((k + 31) / 32));
             transpose_f32_kernel<<<tg, dim3(32, 8), 0, s>>>(Cf, cf_rows, k, cfT.as<float>());
@@ -577,10 +577,10 @@ int mpr_auc_device(const cumf_node *d_R, int64_t nnz, int32_t prob_m, int32_t pr
         CUMF_CUDA(cudaGetLastError());
     }
     // 5. row terms, summed in row order.
-    CUMF_CUDA(mpr.alloc(nseg * 8));
-    CUMF_CUDA(auc.alloc(nseg * 8));
-    CUMF_CUDA(posb.alloc(nseg * 8));
-    CUMF_CUDA(res.alloc(16));
+    CUMF_CUDA(mpr.alloc(nseg * 8, s));
+    CUMF_CUDA(auc.alloc(nseg * 8, s));
+    CUMF_CUDA(posb.alloc(nseg * 8, s));
+    CUMF_CUDA(res.alloc(16, s));
     row_terms_kernel<<<grid_of(nseg), kT, 0, s>>>(seg_off.as<int64_t>(), nseg, spred.as<float>(),
                                                   segcnt.as<unsigned long long>(), cols, mpr.as<double>(),
                                                   auc.as<double>(), posb.as<int64_t>());
@@ -616,9 +616,9 @@ extern "C" int cumf_evaluate(const cumf_problem *te, const cumf_model *model, in
     CUMF_CUDA(cudaStreamCreateWithFlags(&stream.s, cudaStreamNonBlocking));
     DevBuf d_R, d_P, d_Q, d_part, d_sum;
     const size_t pb = (size_t)model->m * model->k * sizeof(float), qb = (size_t)model->n * model->k * sizeof(float);
-    CUMF_CUDA(d_R.alloc(std::max<int64_t>(1, te->nnz) * sizeof(cumf_node)));
-    CUMF_CUDA(d_P.alloc(pb));
-    CUMF_CUDA(d_Q.alloc(qb));
+    CUMF_CUDA(d_R.alloc(std::max<int64_t>(1, te->nnz) * sizeof(cumf_node), stream.s));
+    CUMF_CUDA(d_P.alloc(pb, stream.s));
+    CUMF_CUDA(d_Q.alloc(qb, stream.s));
     if (te->nnz)
         CUMF_CUDA(cudaMemcpyAsync(d_R.p, te->R, te->nnz * sizeof(cumf_node), cudaMemcpyHostToDevice, stream.s));
     if (pb) CUMF_CUDA(cudaMemcpyAsync(d_P.p, model->P, pb, cudaMemcpyHostToDevice, stream.s));
@@ -636,8 +636,8 @@ extern "C" int cumf_evaluate(const cumf_problem *te, const cumf_model *model, in
         *out = (criterion == kRowMPR || criterion == kColMPR) ? two[0] : two[1];
         return CUMF_OK;
     }
-    CUMF_CUDA(d_part.alloc(kBlocks * sizeof(double)));
-    CUMF_CUDA(d_sum.alloc(sizeof(double)));
+    CUMF_CUDA(d_part.alloc(kBlocks * sizeof(double), stream.s));
+    CUMF_CUDA(d_sum.alloc(sizeof(double), stream.s));
     const cumf_node *R = d_R.as<cumf_node>();
     const uint64_t nnz = (uint64_t)te->nnz;
     const float *P = d_P.as<float>(), *Q = d_Q.as<float>();

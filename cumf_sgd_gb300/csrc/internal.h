@@ -55,6 +55,8 @@ inline int64_t batches_per_worker(int64_t nnz, int workers) {
 // Stream-ordered device scratch from a pool of the library that keeps up to 256 MB per device
 // between calls; freed with cudaFreeAsync on the stream of its last use.
 cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t s);
+// Gives the unused part of the pools back to the system.
+void scratch_release();
 
 // ---- sgd_update.cu -------------------------------------------------------------------
 struct Tuning {

@@ -868,7 +868,7 @@ int cumf_user_features(const cumf_node *d_R, int64_t nnz, const float *d_Q, int3
     // degree, rating sum and sum of squares per user.
     const size_t acc_bytes = (size_t)m * k * 4, scratch = acc_bytes + 3 * (size_t)m * 4;
     void *buf = nullptr;
-    CUMF_CUDA(cudaMallocAsync(&buf, scratch, s));
+    CUMF_CUDA(scratch_alloc(&buf, scratch, s));
     float *acc = static_cast<float *>(buf);
     float *deg = acc + (size_t)m * k, *sum = deg + m, *sum2 = sum + m;
     cudaError_t e = cudaMemsetAsync(buf, 0, scratch, s);

@@ -21,6 +21,7 @@
 #include "cumf_sgd.h"
 #include "device_common.cuh"
 #include "internal.h"
+#include "train_common.h"
 
 namespace cumf {
 
@@ -193,18 +194,13 @@ int strata_layout(const cumf_node *d_R, int64_t nnz, int G, cumf_node *d_out, un
                   cudaStream_t s) {
     if (G < 1 || (int64_t)G * G > (1ll << 26)) return fail(CUMF_ERR_ARG, "strata: group count out of range");
     const int64_t blocks = (int64_t)G * G;
-    struct Buf {
-        void *p = nullptr;
-        ~Buf() {
-            if (p) cudaFree(p);
-        }
-    } keys, keys2, idx, idx2, counts, tmp;
+    DevBuf keys, keys2, idx, idx2, counts, tmp;
     const size_t n = (size_t)std::max<int64_t>(1, nnz);
-    CUMF_CUDA(cudaMalloc(&keys.p, n * 4));
-    CUMF_CUDA(cudaMalloc(&keys2.p, n * 4));
-    CUMF_CUDA(cudaMalloc(&idx.p, n * 8));
-    CUMF_CUDA(cudaMalloc(&idx2.p, n * 8));
-    CUMF_CUDA(cudaMalloc(&counts.p, (size_t)(blocks + 1) * 8));
+    CUMF_CUDA(keys.alloc(n * 4, s));
+    CUMF_CUDA(keys2.alloc(n * 4, s));
+    CUMF_CUDA(idx.alloc(n * 8, s));
+    CUMF_CUDA(idx2.alloc(n * 8, s));
+    CUMF_CUDA(counts.alloc((size_t)(blocks + 1) * 8, s));
     unsigned long long *cnt = static_cast<unsigned long long *>(counts.p);
     CUMF_CUDA(cudaMemsetAsync(cnt, 0, (size_t)(blocks + 1) * 8, s));
     const int grid = (int)std::min<int64_t>(65535, (nnz + 255) / 256 + 1);
@@ -220,14 +216,14 @@ int strata_layout(const cumf_node *d_R, int64_t nnz, int G, cumf_node *d_out, un
                                               static_cast<int64_t *>(idx2.p), nnz, 0, end_bit, s));
     size_t tb2 = 0;
     CUMF_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb2, cnt, d_block_off, blocks + 1, s));
-    CUMF_CUDA(cudaMalloc(&tmp.p, std::max(tb, tb2) + 16));
+    CUMF_CUDA(tmp.alloc(std::max(tb, tb2) + 16, s));
     CUMF_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tb, static_cast<uint32_t *>(keys.p),
                                               static_cast<uint32_t *>(keys2.p), static_cast<int64_t *>(idx.p),
                                               static_cast<int64_t *>(idx2.p), nnz, 0, end_bit, s));
     CUMF_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, tb2, cnt, d_block_off, blocks + 1, s));
     gather_records_kernel<<<grid, 256, 0, s>>>(d_R, static_cast<const int64_t *>(idx2.p), nnz, d_out);
     CUMF_CUDA(cudaGetLastError());
-    CUMF_CUDA(cudaStreamSynchronize(s));  // the scratch above is freed on return
+    CUMF_CUDA(cudaStreamSynchronize(s));
     return CUMF_OK;
 }
 

@@ -584,7 +584,7 @@ int parse_text_device(const unsigned char *d_text, int64_t len, int64_t start, c
     // Stream-ordered scratch: block counts, then the total, then the first-bad word, then the
     // block flags of the parse.
     StreamBuf scratch(s);
-    CUMF_CUDA(cudaMallocAsync(&scratch.p, (size_t)(nb + 2) * sizeof(unsigned long long) + (size_t)nb * 4, s));
+    CUMF_CUDA(scratch_alloc(&scratch.p, (size_t)(nb + 2) * sizeof(unsigned long long) + (size_t)nb * 4, s));
     unsigned long long *counts = static_cast<unsigned long long *>(scratch.p);
     unsigned long long *bad = counts + nb + 1;
     uint32_t *flags = reinterpret_cast<uint32_t *>(counts + nb + 2);

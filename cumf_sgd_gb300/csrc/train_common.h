@@ -14,24 +14,42 @@
 
 namespace cumf {
 
-// RAII device buffer.
+// RAII device buffer: alloc(bytes) from cudaMalloc, for buffers that outlive a call; alloc(bytes,
+// stream) stream-ordered from the library's pool, for a call's own work on that stream (the
+// stream outlives the buffer: declare it first).
 struct DevBuf {
     void *p = nullptr;
     size_t bytes = 0;
     DevBuf() = default;
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
-    ~DevBuf() {
-        if (p) cudaFree(p);
-    }
+    ~DevBuf() { release(); }
     cudaError_t alloc(size_t b) {
-        if (p) cudaFree(p);
-        p = nullptr;
+        release();
         bytes = b;
         return cudaMalloc(&p, b ? b : 16);
     }
+    cudaError_t alloc(size_t b, cudaStream_t stream) {
+        release();
+        bytes = b;
+        const cudaError_t e = scratch_alloc(&p, b ? b : 16, stream);
+        if (e != cudaSuccess) p = nullptr;
+        pooled = true;
+        s = stream;
+        return e;
+    }
     template <typename T>
     T *as() const { return reinterpret_cast<T *>(p); }
+
+  private:
+    cudaStream_t s = nullptr;
+    bool pooled = false;
+    void release() {
+        if (p && pooled) cudaFreeAsync(p, s);
+        else if (p) cudaFree(p);
+        p = nullptr;
+        pooled = false;
+    }
 };
 
 struct Stream {

@@ -214,7 +214,9 @@ int cumf_free_model(cumf_model *model);
  * environment; 0 turns the cache off) for the next pinned allocation they fit,
  * because page-locking costs about 30 ms per GB and training calls repeat.  No counterpart
  * in the reference (which leaks its pinned buffers).  This call gives the cached buffers
- * back to the system; buffers still held by problems or models are not affected. */
+ * back to the system; buffers still held by problems or models are not affected.  Device
+ * scratch of the calls below comes from stream-ordered pools that keep up to 256 MB per device
+ * between calls; this call gives their unused part back too. */
 int cumf_release_host_cache(void);
 
 /* ---- rating text (data/netflix/transform.cpp) --------------------------------------- */
