@@ -34,14 +34,6 @@ CUMF_HD int lowest_byte(uint64_t high_bits) {  // index of the lowest byte whose
 #endif
 }
 
-CUMF_HD int popcount64(uint64_t x) {
-#ifdef __CUDA_ARCH__
-    return __popcll(x);
-#else
-    return __builtin_popcountll(x);
-#endif
-}
-
 CUMF_HD bool space_byte(uint32_t c) { return c == 32u || (c - 9u) <= 4u; }
 
 // Bit 7 of byte i is set iff byte i of x is zero.
@@ -72,46 +64,51 @@ CUMF_HD uint32_t digits4(uint32_t d) {
     return (d * 100u + (d >> 16)) & 0xffffu;
 }
 
+// Four characters that are all digits: their low halves; *ok is cleared otherwise.  (A byte is a
+// digit iff its high half is 3 and adding 6 leaves it 3; a carry into the next byte comes only
+// from a byte that is none.)
+CUMF_HD uint32_t digit_values(uint32_t y, bool *ok) {
+    *ok &= ((y & 0xf0f0f0f0u) | (((y + 0x06060606u) & 0xf0f0f0f0u) >> 4)) == 0x33333333u;
+    return y & 0x0f0f0f0fu;
+}
+
+// The number of the first n (0..7) characters of x, all digits; *ok is cleared otherwise.  They
+// are moved to the end of 8 characters, '0' before them.
+CUMF_HD uint32_t digits_value(uint64_t x, int n, bool *ok) {
+    const uint64_t y = n ? (x << (64 - 8 * n)) | ((0x30ull * kOnes) >> (8 * n)) : 0x30ull * kOnes;
+    const uint32_t hi = digit_values((uint32_t)y, ok), lo = digit_values((uint32_t)(y >> 32), ok);
+    return digits4(hi) * 10000u + digits4(lo);
+}
+
 // x: the 8 bytes starting at a token's first character; n (1..7): its length, byte n of x
 // being a space.  is_rating: the token is the third field of a record (%f) rather than an id
 // (%d).  Returns true and the 32-bit field (the id, or the float's bits) when the token is
 // taken here.
 CUMF_HD bool convert_n(uint64_t x, int n, bool is_rating, uint32_t *word) {
-    uint64_t tmh = ((1ull << (8 * n)) - 1) & kHigh;  // bit 7 of each token byte
-    const uint64_t dots = zero_bytes(x ^ (0x2eull * kOnes)) & tmh;
-    // '0' <= b <= '9' per byte: b|0x80 - 0x30 keeps bit 7 iff b >= 0x30; (b&0x7f) + 0x46 sets it
-    // iff b >= 0x3a; bytes >= 0x80 are excluded.
-    const uint64_t digits = ((x | kHigh) - 0x30ull * kOnes) & ~((x & ~kHigh) + 0x46ull * kOnes) & ~x & kHigh;
-    if (tmh & ~(digits | dots)) return false;
-    uint64_t d = x;
-    int nd = n, frac = 0;
-    if (dots) {
-        if (!is_rating || (dots & (dots - 1))) return false;  // '.' in an id, or two of them
-        const uint64_t below = (dots >> 7) - 1;               // the bytes before the '.'
-        d = (x & below) | ((x >> 8) & ~below);                // drop it
-        nd = n - 1;
-        frac = nd - lowest_byte(dots);
-        if (nd == 0) return false;  // "." alone
-    }
-    // Digit values, the last one in byte 7 (leading zero bytes), then two 4-digit halves.
-    const uint64_t dm = (1ull << (8 * nd)) - 1;
-    const uint64_t v = ((d & dm) - (0x30ull * kOnes & dm)) << (64 - 8 * nd);
-    const uint32_t value = digits4((uint32_t)v) * 10000u + digits4((uint32_t)(v >> 32));
+    bool ok = true;
     if (!is_rating) {
-        *word = value;  // < 10^7
-        return true;
+        *word = digits_value(x, n, &ok);  // < 10^7
+        return ok;
+    }
+    int frac = 0;
+    const uint64_t dots = n > 1 ? zero_bytes(x ^ (0x2eull * kOnes)) & ((1ull << (8 * n)) - 1) & kHigh : 0;
+    if (dots) {  // drop the first '.' (a second one is not a digit)
+        const int at = lowest_byte(dots);
+        const uint64_t below = (1ull << (8 * at)) - 1;  // the bytes before it
+        x = (x & below) | ((x >> 8) & ~below);
+        frac = --n - at;
     }
     // value < 10^7 < 2^24 and 10^frac (frac <= 6) are exact floats: one rounded division is
     // the correctly rounded value of value * 10^-frac (the general parser's first case does
     // the same).
-    float f = (float)value;
+    float f = (float)digits_value(x, n, &ok);
     if (frac) f = div_rn(f, ((frac & 1) ? 10.f : 1.f) * ((frac & 2) ? 100.f : 1.f) * ((frac & 4) ? 10000.f : 1.f));
 #ifdef __CUDA_ARCH__
     *word = __float_as_uint(f);
 #else
     memcpy(word, &f, 4);
 #endif
-    return true;
+    return ok;
 }
 
 // The same, finding the token's end in x itself (the first byte below 0x21 must be a space;
