@@ -351,17 +351,23 @@ tc_gemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 // m-block are adjacent, so their A rows are read once from DRAM).  Warp 0 (one lane) streams
 // operand stages through the ring across tile boundaries; warp 1 (one lane) issues the MMAs
 // into one of two tensor-memory accumulators (tile j uses accumulator j % 2) and commits
-// `tfull`; warps 2-5 drain an accumulator (tcgen05.ld, bias, activation, staged coalesced
-// stores) and release it through `tempty` while the next tile's MMAs fill the other one.
-constexpr int kPersThreads = 192;
+// `tfull`; warps 2-17 drain an accumulator (tcgen05.ld, bias, activation, staged coalesced
+// stores), four to a tensor-memory lane quarter, and release it through `tempty` while the next
+// tile's MMAs fill the other one.  The epilogue is what bounds it (an activation is some fifty
+// instructions per output): at 50,000 x 512 outputs with gelu four epilogue warps took 85 us per
+// product, eight 53, sixteen 46.  Their staging blocks take one stage of the 256-wide ring and
+// two of the 128-wide one, which K of a few stages does not miss.
+constexpr int kPersEpilogueWarps = 16;
+constexpr int kPersThreads = 64 + 32 * kPersEpilogueWarps;
 
 template <int BN, int kStages>
 struct PersSmem {
     static constexpr int A_BYTES = kTcBM * 128;
     static constexpr int B_BYTES = BN * 128;
     static constexpr int STAGE = A_BYTES + B_BYTES;
-    static constexpr int STG = 4 * 32 * kStgStride * 4;  // four epilogue warps' staging blocks
+    static constexpr int STG = kPersEpilogueWarps * 32 * kStgStride * 4;  // the epilogue warps' staging blocks
     static constexpr int TOTAL = 1024 + kStages * STAGE + STG + 256;
+    static_assert(TOTAL <= 232448, "shared memory of one CTA");
 };
 
 __device__ __forceinline__ bool aborted(const int *flag) { return *reinterpret_cast<const volatile int *>(flag) != 0; }
@@ -398,7 +404,8 @@ tc_gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
         }
         for (int i = 0; i < 2; ++i) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&tfull[i])));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;\n" ::"r"(smem_u32(&tempty[i])));  // one per epilogue warp
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&tempty[i])),
+                         "n"(kPersEpilogueWarps));  // one arrival per epilogue warp
         }
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(mma_done)));
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -483,8 +490,9 @@ tc_gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
                              smem_u32(mma_done))
                          : "memory");
         }
-    } else {  // epilogue warps 2-5: tensor-memory lanes 32 (warp % 4)..
-        const int quarter = warp & 3;
+    } else {  // epilogue warps: tensor-memory lanes 32 (warp % 4).., a quarter of the columns each
+        const int quarter = warp & 3, part = (warp - 2) >> 2;
+        constexpr int kCols = BN / (kPersEpilogueWarps / 4);
         float *stg = stg_all + (warp - 2) * (32 * kStgStride);
         for (int j = 0; j < my_tiles; ++j) {
             const int acc = j & 1;
@@ -498,7 +506,7 @@ tc_gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             }
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const int r0 = tm * kTcBM + quarter * 32, n0 = tn * BN;
-            for (int c0 = 0; c0 < BN && n0 + c0 < N; c0 += 32) {
+            for (int c0 = part * kCols; c0 < (part + 1) * kCols && n0 + c0 < N; c0 += 32) {
                 uint32_t r[32];
                 const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN + c0);
                 asm volatile(
@@ -649,8 +657,8 @@ cudaError_t launch_tc_gemm(const void *A, const void *B, int M, int N, int K, co
     // next tiles' loads and MMAs.
     if (splits == 1 && sms > 0 && (long long)tiles_m * tiles_n >= 2ll * sms) {
         const int g = std::min(tiles_m * tiles_n, sms);
-        return wide ? launch_persistent<256, 4>(g, ma, mb, M, N, K, bias, act, out, out_f32, ldo, pre_out, status, s)
-                    : launch_persistent<128, 6>(g, ma, mb, M, N, K, bias, act, out, out_f32, ldo, pre_out, status, s);
+        return wide ? launch_persistent<256, 3>(g, ma, mb, M, N, K, bias, act, out, out_f32, ldo, pre_out, status, s)
+                    : launch_persistent<128, 4>(g, ma, mb, M, N, K, bias, act, out, out_f32, ldo, pre_out, status, s);
     }
     const dim3 grid(tiles_m, tiles_n, splits);
     if (wide)
