@@ -81,14 +81,16 @@ __global__ void user_qsum_kernel(const cumf_node *R, int64_t nnz, int32_t m, int
 }
 
 // Sort keys of the ratings: the user, or m for a rating outside [0, m) x [0, n) (sorted last
-// and left out); values: the rating's index.
+// and left out); values: the rating and its item's bits, which travel with the key (the sort of
+// 5.2 M pairs took 141 us with 8-byte values as with 4-byte indices), so that what follows reads
+// them in order instead of gathering the records.
 __global__ void user_keys_kernel(const cumf_node *R, uint32_t nnz, int32_t m, int32_t n, uint32_t *key,
-                                 uint32_t *idx) {
+                                 float2 *val) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += gridDim.x * blockDim.x) {
         const cumf_node x = R[i];
         const bool ok = (uint32_t)x.u < (uint32_t)m && (uint32_t)x.v < (uint32_t)n;
         key[i] = ok ? (uint32_t)x.u : (uint32_t)m;
-        idx[i] = i;
+        val[i] = make_float2(x.r, __int_as_float(x.v));
     }
 }
 
@@ -105,24 +107,47 @@ __global__ void user_segments_kernel(const uint32_t *key, uint32_t nnz, int32_t 
     }
 }
 
+// V consecutive floats in one load (the caller checks the alignment).
+template <int V>
+__device__ __forceinline__ void load_cols(float (&dst)[V], const float *src) {
+    if constexpr (V == 4) {
+        const float4 x = __ldg(reinterpret_cast<const float4 *>(src));
+        dst[0] = x.x, dst[1] = x.y, dst[2] = x.z, dst[3] = x.w;
+    } else if constexpr (V == 2) {
+        const float2 x = __ldg(reinterpret_cast<const float2 *>(src));
+        dst[0] = x.x, dst[1] = x.y;
+    } else {
+        dst[0] = __ldg(src);
+    }
+}
+
 // One warp per user over the user's ratings in their original order (a stable sort by user):
 // the rating sum and sum of squares by a fixed-order warp reduction, then
-// sum (r - mean) q / deg accumulated rating by rating in registers, 32 * KPL columns per
-// pass; X[u] = (that sum, log(1 + deg)/4, (mean - 3)/2, var/2).  The ratings are fetched 32
-// at a time (one per lane, then broadcast) and the item rows of four ratings are loaded
-// before they are added, in rating order.  No atomics: the features are the same bits on
-// every run.
-template <int KPL>
-__global__ void user_rows_kernel(const cumf_node *R, const uint32_t *order, const int64_t *seg, int32_t m,
-                                 const float *Q, int k, float *X, int ldx) {
+// sum (r - mean) q / deg accumulated rating by rating in registers; X[u] = (that sum,
+// log(1 + deg)/4, (mean - 3)/2, var/2).  A lane owns V consecutive columns (one load of V
+// floats per rating) in each of G groups, 32 V G columns per pass.  The ratings are fetched 32
+// at a time (one per lane, then broadcast), the next 32 while these are used; the item rows of
+// four ratings are loaded before they are added, in rating order.  No atomics: the features
+// are the same bits on every run and for every V and G.
+//
+// Bound by the item rows out of L2 (512 bytes per rating at 128 columns).  5.2 M ratings, 50,000
+// users, 128 columns: 360 us with the records gathered through a sorted index and four
+// loads of one float per rating, 150 us so; eight rows in flight are no faster.
+template <int V, int G>
+__global__ void __launch_bounds__(kT) user_rows_kernel(const float2 *val, const int64_t *seg, int32_t m,
+                                                       const float *Q, int k, float *X, int ldx) {
+    constexpr int F = 4;
     const int lane = threadIdx.x & 31;
     const int64_t w0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t u = w0; u < m; u += nw) {
-        const int64_t a = seg[u], b = seg[u + 1];
+        const int64_t a = seg[u];
+        const uint32_t cnt = (uint32_t)(seg[u + 1] - a);
+        const float2 *row = val + a;
         float s = 0.f, s2 = 0.f;
-        for (int64_t t = a + lane; t < b; t += 32) {
-            const float r = R[order[t]].r;
+#pragma unroll 4
+        for (uint32_t t = lane; t < cnt; t += 32) {
+            const float r = row[t].x;
             s += r;
             s2 += r * r;
         }
@@ -130,53 +155,80 @@ __global__ void user_rows_kernel(const cumf_node *R, const uint32_t *order, cons
             s += __shfl_xor_sync(0xffffffffu, s, o);
             s2 += __shfl_xor_sync(0xffffffffu, s2, o);
         }
-        const float d = (float)(b - a);
-        const float mean = d > 0 ? s / d : 0.f;
+        const float d = (float)cnt;
+        const float mean = cnt > 0 ? s / d : 0.f;
         float *xu = X + u * ldx;
-        for (int c0 = 0; c0 < k; c0 += 32 * KPL) {
-            float acc[KPL];
+        for (int c0 = 0; c0 < k; c0 += 32 * V * G) {
+            const int cl = c0 + lane * V;  // this lane's first column; a group is 32 V further
+            float acc[G][V];
+            const float *q0[G];
 #pragma unroll
-            for (int j = 0; j < KPL; ++j) acc[j] = 0.f;
-            bool col[KPL];
+            for (int g = 0; g < G; ++g) {
+                q0[g] = Q + (cl + g * 32 * V < k ? cl + g * 32 * V : 0);  // a lane past k loads column 0, unused
 #pragma unroll
-            for (int j = 0; j < KPL; ++j) col[j] = c0 + lane + 32 * j < k;
-            for (int64_t t0 = a; t0 < b; t0 += 32) {
-                float cl = 0.f;
-                int vl = 0;
-                if (t0 + lane < b) {
-                    const cumf_node x = R[order[t0 + lane]];
-                    cl = (x.r - s / d) / d;
-                    vl = x.v;
-                }
-                const int cnt = (int)(b - t0 < 32 ? b - t0 : 32);
-                for (int j0 = 0; j0 < cnt; j0 += 4) {
-                    float c4[4], q4[4][KPL];
+                for (int j = 0; j < V; ++j) acc[g][j] = 0.f;
+            }
+            float2 next = make_float2(0.f, 0.f);
+            if ((uint32_t)lane < cnt) next = row[lane];
+            for (uint32_t t0 = 0; t0 < cnt; t0 += 32) {
+                const float c = (next.x - s / d) / d;
+                const int item = __float_as_int(next.y);
+                if (cnt - t0 > 32 + (uint32_t)lane) next = row[t0 + 32 + lane];
+                const int some = (int)(cnt - t0 < 32 ? cnt - t0 : 32);
+                float c4[F], q[F][G][V];
+                int j0 = 0;
+                for (; j0 + F <= some; j0 += F) {
 #pragma unroll
-                    for (int h = 0; h < 4; ++h) {
-                        c4[h] = __shfl_sync(0xffffffffu, cl, (j0 + h) & 31);
-                        const int v = __shfl_sync(0xffffffffu, vl, (j0 + h) & 31);
-                        const float *q = Q + (int64_t)v * k + c0 + lane;
+                    for (int h = 0; h < F; ++h) {
+                        c4[h] = __shfl_sync(0xffffffffu, c, j0 + h);
+                        const int64_t at = (int64_t)__shfl_sync(0xffffffffu, item, j0 + h) * k;
 #pragma unroll
-                        for (int j = 0; j < KPL; ++j) q4[h][j] = (j0 + h < cnt && col[j]) ? q[32 * j] : 0.f;
+                        for (int g = 0; g < G; ++g) load_cols<V>(q[h][g], q0[g] + at);
                     }
 #pragma unroll
-                    for (int h = 0; h < 4; ++h)
-                        if (j0 + h < cnt) {
+                    for (int h = 0; h < F; ++h)
 #pragma unroll
-                            for (int j = 0; j < KPL; ++j) acc[j] += c4[h] * q4[h][j];
-                        }
+                        for (int g = 0; g < G; ++g)
+#pragma unroll
+                            for (int j = 0; j < V; ++j) acc[g][j] += c4[h] * q[h][g][j];
+                }
+                for (; j0 < some; ++j0) {
+                    c4[0] = __shfl_sync(0xffffffffu, c, j0);
+                    const int64_t at = (int64_t)__shfl_sync(0xffffffffu, item, j0) * k;
+#pragma unroll
+                    for (int g = 0; g < G; ++g) {
+                        load_cols<V>(q[0][g], q0[g] + at);
+#pragma unroll
+                        for (int j = 0; j < V; ++j) acc[g][j] += c4[0] * q[0][g][j];
+                    }
                 }
             }
 #pragma unroll
-            for (int j = 0; j < KPL; ++j)
-                if (col[j]) xu[c0 + lane + 32 * j] = acc[j];
+            for (int g = 0; g < G; ++g)
+                if (cl + g * 32 * V < k) {
+#pragma unroll
+                    for (int j = 0; j < V; ++j) xu[cl + g * 32 * V + j] = acc[g][j];
+                }
         }
         if (lane == 0) {
             xu[k] = logf(1.f + d) * 0.25f;
-            xu[k + 1] = d > 0 ? (mean - 3.f) * 0.5f : 0.f;
-            xu[k + 2] = (d > 0 ? fmaxf(s2 / d - mean * mean, 0.f) : 0.f) * 0.5f;
+            xu[k + 1] = cnt > 0 ? (mean - 3.f) * 0.5f : 0.f;
+            xu[k + 2] = (cnt > 0 ? fmaxf(s2 / d - mean * mean, 0.f) : 0.f) * 0.5f;
         }
     }
+}
+
+// The widest load that every row of Q allows (k and the base a multiple of it) and that still
+// gives most lanes a column: 4 floats from 65 columns on, 2 from 33 on.
+void launch_user_rows(int grid, const float2 *val, const int64_t *seg, int32_t m, const float *Q, int k, float *X,
+                      cudaStream_t s) {
+    auto can = [&](int v) { return k % v == 0 && reinterpret_cast<uintptr_t>(Q) % (4 * v) == 0; };
+    if (k > 128 && can(4)) user_rows_kernel<4, 2><<<grid, kT, 0, s>>>(val, seg, m, Q, k, X, k + 3);
+    else if (k > 64 && can(4)) user_rows_kernel<4, 1><<<grid, kT, 0, s>>>(val, seg, m, Q, k, X, k + 3);
+    else if (k > 32 && k <= 64 && can(2)) user_rows_kernel<2, 1><<<grid, kT, 0, s>>>(val, seg, m, Q, k, X, k + 3);
+    else if (k <= 32) user_rows_kernel<1, 1><<<grid, kT, 0, s>>>(val, seg, m, Q, k, X, k + 3);
+    else if (k <= 64) user_rows_kernel<1, 2><<<grid, kT, 0, s>>>(val, seg, m, Q, k, X, k + 3);
+    else user_rows_kernel<1, 4><<<grid, kT, 0, s>>>(val, seg, m, Q, k, X, k + 3);
 }
 
 // x[u] = (acc[u][0:k], log(1 + deg)/4, (mean - 3)/2, var/2) for the m users (ldx = k + 3).
@@ -517,10 +569,10 @@ int mlp_refresh(Mlp *mp, cudaStream_t s) {
 }
 
 // Forward over rows [0, rows) of X (fp32, rows x d_in; with perm, row r is X[perm[*batch_idx *
-// batch + r]]); Y (fp32 rows x d_out) in mp->y.  train: also X's bf16 transpose and the
+// batch + r]]); Y (fp32 rows x d_out) in Y, or with its padding rows in mp->y.  train: also X's bf16 transpose and the
 // pre-activations, which the backward pass uses.
 int mlp_forward_ws(Mlp *mp, const float *X, int64_t rows, cudaStream_t s, bool train, const int32_t *perm = nullptr,
-                   const int *batch_idx = nullptr, int64_t batch = 0) {
+                   const int *batch_idx = nullptr, int64_t batch = 0, float *Y = nullptr) {
     if (int rc = mlp_ensure(mp, rows, train)) return rc;
     const float *P = mp->params.as<float>();
     const int h = mp->h;
@@ -533,8 +585,8 @@ int mlp_forward_ws(Mlp *mp, const float *X, int64_t rows, cudaStream_t s, bool t
                              train ? mp->pre1.as<float>() : nullptr, st, s));
     CUMF_CUDA(launch_tc_gemm(mp->h1.p, mp->w2b.p, (int)rp, h, h, P + mp->off_b2, 1, mp->h2.p, 0, h,
                              train ? mp->pre2.as<float>() : nullptr, st, s));
-    CUMF_CUDA(launch_tc_gemm(mp->h2.p, mp->w3b.p, (int)rp, mp->d_out, h, P + mp->off_b3, 0, mp->y.p, 1, mp->d_out,
-                             nullptr, st, s));
+    CUMF_CUDA(launch_tc_gemm(mp->h2.p, mp->w3b.p, (int)(Y ? rows : rp), mp->d_out, h, P + mp->off_b3, 0,
+                             Y ? Y : mp->y.as<float>(), 1, mp->d_out, nullptr, st, s));
     return CUMF_OK;
 }
 
@@ -674,8 +726,8 @@ int cumf_mlp_forward(void *mlp, const float *d_X, int64_t rows, float *d_Y, void
     const int64_t chunk = 1 << 16;
     for (int64_t r0 = 0; r0 < rows; r0 += chunk) {
         const int64_t r = std::min(chunk, rows - r0);
-        if (int rc = mlp_forward_ws(mp, d_X + r0 * mp->d_in, r, s, false)) return rc;
-        CUMF_CUDA(cudaMemcpyAsync(d_Y + r0 * mp->d_out, mp->y.p, r * mp->d_out * 4, cudaMemcpyDeviceToDevice, s));
+        if (int rc = mlp_forward_ws(mp, d_X + r0 * mp->d_in, r, s, false, nullptr, nullptr, 0, d_Y + r0 * mp->d_out))
+            return rc;
     }
     return mlp_check_status(mp, s);
 }
@@ -822,39 +874,37 @@ int cumf_user_features(const cumf_node *d_R, int64_t nnz, const float *d_Q, int3
         return fail(CUMF_ERR_ARG, "user_features: bad arguments");
     cudaStream_t s = (cudaStream_t)stream;
     if (nnz < 0xffffffffll && m < 0x7fffffff) {
-        // The ratings stably sorted by user (32-bit keys and indices), then one warp per user.
+        // The ratings stably sorted by user (32-bit keys), then one warp per user.
         const uint32_t N = (uint32_t)nnz;
         int end_bit = 1;
         while (end_bit < 32 && ((uint32_t)m >> end_bit) != 0) ++end_bit;
-        size_t tmp_bytes = 0;
-        CUMF_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, (const uint32_t *)nullptr, (uint32_t *)nullptr,
-                                                  (const uint32_t *)nullptr, (uint32_t *)nullptr, N, 0, end_bit, s));
         auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
-        const size_t kb = up((size_t)N * 4 + 4), sb = up(((size_t)m + 1) * 8);
+        const size_t kb = up((size_t)N * 4 + 4), vb = up((size_t)N * 8 + 8), sb = up(((size_t)m + 1) * 8);
+        cub::DoubleBuffer<uint32_t> key(nullptr, nullptr);
+        cub::DoubleBuffer<float2> val(nullptr, nullptr);
+        size_t tmp_bytes = 0;
+        CUMF_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, key, val, N, 0, end_bit, s));
         void *buf = nullptr;
-        CUMF_CUDA(scratch_alloc(&buf, 4 * kb + sb + up(tmp_bytes), s));
+        CUMF_CUDA(scratch_alloc(&buf, 2 * kb + 2 * vb + sb + up(tmp_bytes), s));
         char *p = static_cast<char *>(buf);
-        uint32_t *key = reinterpret_cast<uint32_t *>(p), *idx = reinterpret_cast<uint32_t *>(p + kb);
-        uint32_t *key2 = reinterpret_cast<uint32_t *>(p + 2 * kb), *idx2 = reinterpret_cast<uint32_t *>(p + 3 * kb);
-        int64_t *seg = reinterpret_cast<int64_t *>(p + 4 * kb);
-        void *tmp = p + 4 * kb + sb;
+        key.d_buffers[0] = reinterpret_cast<uint32_t *>(p);
+        key.d_buffers[1] = reinterpret_cast<uint32_t *>(p + kb);
+        val.d_buffers[0] = reinterpret_cast<float2 *>(p + 2 * kb);
+        val.d_buffers[1] = reinterpret_cast<float2 *>(p + 2 * kb + vb);
+        int64_t *seg = reinterpret_cast<int64_t *>(p + 2 * kb + 2 * vb);
+        void *tmp = p + 2 * kb + 2 * vb + sb;
         cudaError_t e = cudaSuccess;
         if (N > 0) {
-            user_keys_kernel<<<grid_of(N), kT, 0, s>>>(d_R, N, m, n, key, idx);
+            user_keys_kernel<<<grid_of(N), kT, 0, s>>>(d_R, N, m, n, key.Current(), val.Current());
             e = cudaGetLastError();
-            if (e == cudaSuccess)
-                e = cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, key, key2, idx, idx2, N, 0, end_bit, s);
+            if (e == cudaSuccess) e = cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, key, val, N, 0, end_bit, s);
         }
         if (e == cudaSuccess) {
-            user_segments_kernel<<<grid_of((int64_t)m + 1), kT, 0, s>>>(key2, N, m, seg);
+            user_segments_kernel<<<grid_of((int64_t)m + 1), kT, 0, s>>>(key.Current(), N, m, seg);
             e = cudaGetLastError();
         }
         if (e == cudaSuccess) {
-            const int g = grid_of((int64_t)m * 32);
-            if (k <= 32) user_rows_kernel<1><<<g, kT, 0, s>>>(d_R, idx2, seg, m, d_Q, k, d_X, k + 3);
-            else if (k <= 64) user_rows_kernel<2><<<g, kT, 0, s>>>(d_R, idx2, seg, m, d_Q, k, d_X, k + 3);
-            else if (k <= 128) user_rows_kernel<4><<<g, kT, 0, s>>>(d_R, idx2, seg, m, d_Q, k, d_X, k + 3);
-            else user_rows_kernel<8><<<g, kT, 0, s>>>(d_R, idx2, seg, m, d_Q, k, d_X, k + 3);
+            launch_user_rows(grid_of((int64_t)m * 32), val.Current(), seg, m, d_Q, k, d_X, s);
             e = cudaGetLastError();
         }
         const cudaError_t ef = cudaFreeAsync(buf, s);
