@@ -24,12 +24,10 @@
 #include "cumf_sgd.h"
 #include "internal.h"
 #include "rng.h"
+#include "tc_gemm.h"
 #include "train_common.h"
 
 namespace cumf {
-
-cudaError_t launch_tc_gemm(const void *A, const void *B, int M, int N, int K, const float *bias, int act,
-                           void *out, int out_f32, int ldo, float *pre_out, int *status, cudaStream_t s);
 
 namespace {
 
@@ -253,15 +251,13 @@ __global__ void user_finish_kernel(int32_t m, int k, const float *acc, const flo
     }
 }
 
-// ---- elementwise helpers ---------------------------------------------------------------
-
 // ---- 32 x 32 tile kernels: an elementwise result written row-major and transposed --------
 //
-// The weight-gradient products dW = dZ^T A take both operands K-major (K = the batch rows), so
-// every bf16 activation or gradient that feeds one is also needed transposed.  The kernels
-// below produce both copies from one read of their inputs: a block computes a 32 x 32 tile,
-// writes it row-major, stages it in shared memory (fp32, conflict-free) and writes the
-// transpose; gradient tiles also leave their 32-row column sums for the bias gradient.
+// The weight-gradient products dW = dZ^T A take both operands K-major (K = the batch rows), and
+// the products dA = dZ W take W transposed, so the batch's features and the bf16 weights are
+// needed row-major and transposed (activations and their gradients get both copies from the
+// products' epilogues).  A block computes a 32 x 32 tile, writes it row-major, stages it in shared
+// memory (fp32, conflict-free) and writes the transpose.
 constexpr int kTile = 32;
 constexpr int kTileRows = 8;  // threads per column of a tile (blockDim = 32 x 8)
 
@@ -274,20 +270,9 @@ __device__ __forceinline__ void store_tile_t(const float (*tile)[kTile + 1], __n
     }
 }
 
-// partial[tile row][c] = the tile's column c summed over its 32 rows: each thread's own rows
-// (y, y + 8, y + 16, y + 24, in order, in `mine`), then the 8 thread sums in order.  Call after
-// a barrier that follows the writes of lanes[][] (lanes[threadIdx.y][threadIdx.x] = mine).
-__device__ __forceinline__ void tile_colsum(const float (*lanes)[kTile + 1], float *partial, int cols, int c0) {
-    if (threadIdx.y == 0 && c0 + (int)threadIdx.x < cols) {
-        float sum = 0.f;
-        for (int y = 0; y < kTileRows; ++y) sum += lanes[y][threadIdx.x];
-        partial[(int64_t)blockIdx.x * cols + c0 + threadIdx.x] = sum;
-    }
-}
-
 // D (rp x ldd bf16) and, when Dt != NULL, Dt (ldd x rp) from the fp32 rows of S (cols wide):
 // row r < valid is S[perm[*batch_idx * batch + r]] (perm NULL: S[r]); other rows and the
-// columns cols..ldd are zero.
+// columns cols..ldd are zero.  With F instead of D, the valid rows as fp32 (ldd wide).
 struct ConvertJob {
     const float *S;
     int cols;
@@ -296,12 +281,15 @@ struct ConvertJob {
     int64_t batch;
     int valid, rp, ldd;
     __nv_bfloat16 *D, *Dt;
+    float *F;
 };
 struct ConvertJobs {
     ConvertJob job[3];  // blockIdx.z picks one; tiles outside its rp x ldd return
+    int64_t *step;      // not NULL: Adam's step count, which this launch advances
 };
 
 __global__ void __launch_bounds__(kTile * kTileRows) convert_t_kernel(const __grid_constant__ ConvertJobs jobs) {
+    if (jobs.step && (blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x | threadIdx.y) == 0) ++*jobs.step;
     const ConvertJob &jb = jobs.job[blockIdx.z];
     const float *S = jb.S;
     const int cols = jb.cols, valid = jb.valid, rp = jb.rp, ldd = jb.ldd;
@@ -315,6 +303,10 @@ __global__ void __launch_bounds__(kTile * kTileRows) convert_t_kernel(const __gr
         float v = 0.f;
         if (r < valid && c < cols) v = S[(int64_t)(idx ? idx[r] : r) * cols + c];
         const __nv_bfloat16 b = __float2bfloat16_rn(v);
+        if (jb.F) {
+            if (r < valid && c < cols) jb.F[(int64_t)r * ldd + c] = v;
+            continue;
+        }
         if (r < rp && c < ldd) D[(int64_t)r * ldd + c] = b;
         tile[j][threadIdx.x] = __bfloat162float(b);
     }
@@ -323,139 +315,144 @@ __global__ void __launch_bounds__(kTile * kTileRows) convert_t_kernel(const __gr
     store_tile_t(tile, Dt, rp, r0, c0, rp, ldd);
 }
 
-// D^T (cols x rows) of a bf16 matrix D (rows x cols).
-__global__ void __launch_bounds__(kTile * kTileRows) transpose_t_kernel(const __nv_bfloat16 *D, int rows, int cols,
-                                                                        __nv_bfloat16 *Dt) {
+struct Adam {
+    float *w, *m1, *m2;
+    float lr, b1, b2, eps;
+    const int64_t *step;  // t, the number of this step; NULL: gradients only
+};
+
+// Adam's update of element i (value w, moments m1 and m2) with gradient g; returns the new
+// value.  c1, c2: 1 - b1^t, 1 - b2^t.
+__device__ __forceinline__ float adam_element(const Adam &ad, int64_t i, float g, float w, float m1, float m2,
+                                              float c1, float c2) {
+    const float a = ad.b1 * m1 + (1.f - ad.b1) * g;
+    const float b = ad.b2 * m2 + (1.f - ad.b2) * g * g;
+    ad.m1[i] = a;
+    ad.m2[i] = b;
+    w -= ad.lr * (a / c1) / (sqrtf(b / c2) + ad.eps);
+    ad.w[i] = w;
+    return w;
+}
+
+// What follows a step's products: the weight gradients' K parts and the bias gradients' tile
+// sums added (in order), the gradients stored, Adam's update, the bf16 copies and transposes of
+// the new weights, and the loss.  Blocks first[l].. take the 32 x 32 tiles of weight l, blocks
+// first[3 + l].. 32 columns of bias l, the last block the loss and the device state.
+struct FinishWeight {
+    const float *part;  // [splits][rows][ld]
+    int64_t off;
+    int rows, cols, ld;  // ld >= cols: the padded columns of W1 are left out
+    __nv_bfloat16 *b, *bt;
+};
+struct FinishBias {
+    const float *part;  // [tiles][cols]
+    int64_t off;
+    int cols;
+};
+struct FinishArgs {
+    FinishWeight w[3];
+    FinishBias bias[3];
+    int first[7];
+    int splits, tiles;  // parts of a weight gradient, of a bias gradient
+    float *grads;
+    Adam adam;
+    const double *loss_part;
+    int loss_parts;
+    double *loss, *loss_sum;
+    int *batch_idx;  // advanced, and loss added to loss_sum, where not NULL
+};
+
+__global__ void __launch_bounds__(kTile * kTileRows) finish_step_kernel(const __grid_constant__ FinishArgs args) {
     __shared__ float tile[kTile][kTile + 1];
-    const int r0 = blockIdx.x * kTile, c0 = blockIdx.y * kTile;
-    for (int j = threadIdx.y; j < kTile; j += kTileRows) {
-        const int r = r0 + j, c = c0 + threadIdx.x;
-        tile[j][threadIdx.x] = (r < rows && c < cols) ? __bfloat162float(D[(int64_t)r * cols + c]) : 0.f;
-    }
-    __syncthreads();
-    store_tile_t(tile, Dt, rows, r0, c0, rows, cols);
-}
-
-__device__ __forceinline__ float gelu_grad(float x) {
-    const float c = 0.7978845608028654f;
-    const float u = c * (x + 0.044715f * x * x * x);
-    const float t = tanhf(u);
-    return 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * c * (1.f + 3.f * 0.044715f * x * x);
-}
-
-// dZ = dA * gelu'(pre) -> bf16 (rows beyond `valid` zero), its transpose dZt, and the tile
-// column sums of dZ (the bias gradient's partial sums).
-__global__ void __launch_bounds__(kTile * kTileRows) gelu_back_t_kernel(const float *dA, const float *pre, int rp,
-                                                                        int valid, int cols, __nv_bfloat16 *dZ,
-                                                                        __nv_bfloat16 *dZt, float *partial) {
-    __shared__ float tile[kTile][kTile + 1];
-    __shared__ float lanes[kTileRows][kTile + 1];
-    const int r0 = blockIdx.x * kTile, c0 = blockIdx.y * kTile;
-    float mine = 0.f;
-    for (int j = threadIdx.y; j < kTile; j += kTileRows) {
-        const int r = r0 + j, c = c0 + threadIdx.x;
-        const int64_t i = (int64_t)r * cols + c;
-        const float g = (r < valid && c < cols) ? dA[i] * gelu_grad(pre[i]) : 0.f;
-        const __nv_bfloat16 b = __float2bfloat16_rn(g);
-        if (r < rp && c < cols) dZ[i] = b;
-        const float bv = __bfloat162float(b);
-        tile[j][threadIdx.x] = bv;
-        mine += bv;
-    }
-    lanes[threadIdx.y][threadIdx.x] = mine;
-    __syncthreads();
-    tile_colsum(lanes, partial, cols, c0);
-    store_tile_t(tile, dZt, rp, r0, c0, rp, cols);
-}
-
-// dY = 2 (Y - T) / B (bf16, zero for padding rows), its transpose, the tile column sums and
-// the loss (sum of squared errors).  Row r < valid of T is T[perm[*batch_idx * batch + r]]
-// (perm NULL: T[r]).
-__global__ void __launch_bounds__(kTile * kTileRows) mse_grad_t_kernel(const float *Y, const float *T,
-                                                                       const int32_t *perm, const int *batch_idx,
-                                                                       int64_t batch, int rp, int valid, int cols,
-                                                                       float inv_b, __nv_bfloat16 *dY,
-                                                                       __nv_bfloat16 *dYt, float *partial,
-                                                                       double *loss) {
-    __shared__ float tile[kTile][kTile + 1];
-    __shared__ float lanes[kTileRows][kTile + 1];
-    __shared__ double s_loss[kTileRows];
-    const int r0 = blockIdx.x * kTile, c0 = blockIdx.y * kTile;
-    const int32_t *idx = perm ? perm + (int64_t)*batch_idx * batch : nullptr;
-    double acc = 0;
-    float mine = 0.f;
-    for (int j = threadIdx.y; j < kTile; j += kTileRows) {
-        const int r = r0 + j, c = c0 + threadIdx.x;
-        float g = 0.f;
-        if (r < valid && c < cols) {
-            const float d = Y[(int64_t)r * cols + c] - T[(int64_t)(idx ? idx[r] : r) * cols + c];
-            acc += (double)d * d;
-            g = 2.f * d * inv_b;
-        }
-        const __nv_bfloat16 b = __float2bfloat16_rn(g);
-        if (r < rp && c < cols) dY[(int64_t)r * cols + c] = b;
-        const float bv = __bfloat162float(b);
-        tile[j][threadIdx.x] = bv;
-        mine += bv;
-    }
-    lanes[threadIdx.y][threadIdx.x] = mine;
-    for (int o = 16; o >= 1; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (threadIdx.x == 0) s_loss[threadIdx.y] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0 && threadIdx.y == 0 && loss) {
-        double t = 0;
-        for (int w = 0; w < kTileRows; ++w) t += s_loss[w];
-        atomicAdd(loss, t);
-    }
-    tile_colsum(lanes, partial, cols, c0);
-    store_tile_t(tile, dYt, rp, r0, c0, rp, cols);
-}
-
-// Bias gradient: out[c] = the tile column sums of column c (tile_colsum).  Block: 32 columns x
-// 8 lanes; lane y adds tiles y, y + 8, ... in order, then the 8 lane sums are added in order.
-__global__ void __launch_bounds__(kTile * kTileRows) colsum_finish_kernel(const float *partial, int tiles, int cols,
-                                                                          float *out) {
-    __shared__ float lanes[kTileRows][kTile + 1];
-    const int c = blockIdx.x * kTile + threadIdx.x;
-    float sum = 0.f;
-    if (c < cols)
-        for (int t = threadIdx.y; t < tiles; t += kTileRows) sum += partial[(int64_t)t * cols + c];
-    lanes[threadIdx.y][threadIdx.x] = sum;
-    __syncthreads();
-    if (threadIdx.y == 0 && c < cols) {
-        float total = 0.f;
-        for (int y = 0; y < kTileRows; ++y) total += lanes[y][threadIdx.x];
-        out[c] = total;
-    }
-}
-
-// After a step: the next batch of the permutation, Adam's step count, the step's loss added to
-// the epoch's.  One thread; this state lives on the device so that a captured step can replay.
-__global__ void step_end_kernel(int64_t *step, int *batch_idx, const double *loss, double *loss_sum) {
-    ++*step;
-    ++*batch_idx;
-    *loss_sum += *loss;
-}
-
-// Adam step number *step + 1 (bias corrections 1 - b^t computed once per block).
-__global__ void adam_kernel(float *w, const float *g, float *m1, float *m2, int64_t n, float lr, float b1, float b2,
-                            float eps, const int64_t *step) {
     __shared__ float corr[2];
-    if (threadIdx.x == 0) {
-        const float t = (float)(*step + 1);
-        corr[0] = 1.f - powf(b1, t);
-        corr[1] = 1.f - powf(b2, t);
+    __shared__ double sums[kTileRows];
+    const int bx = (int)blockIdx.x, tx = threadIdx.x, ty = threadIdx.y;
+    const bool adam = args.adam.step != nullptr;
+    if (adam && tx == 0 && ty == 0) {
+        const float t = (float)*args.adam.step;
+        corr[0] = 1.f - powf(args.adam.b1, t);
+        corr[1] = 1.f - powf(args.adam.b2, t);
     }
     __syncthreads();
     const float c1 = corr[0], c2 = corr[1];
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const float gi = g[i];
-        const float a = b1 * m1[i] + (1.f - b1) * gi;
-        const float b = b2 * m2[i] + (1.f - b2) * gi * gi;
-        m1[i] = a;
-        m2[i] = b;
-        w[i] -= lr * (a / c1) / (sqrtf(b / c2) + eps);
+    if (bx >= args.first[6]) {  // loss
+        double acc = 0;
+        for (int i = ty * kTile + tx; i < args.loss_parts; i += kTile * kTileRows) acc += args.loss_part[i];
+        for (int o = 16; o >= 1; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (tx == 0) sums[ty] = acc;
+        __syncthreads();
+        if (tx == 0 && ty == 0) {
+            double total = 0;
+            for (int y = 0; y < kTileRows; ++y) total += sums[y];
+            *args.loss = total;
+            if (args.batch_idx) {
+                ++*args.batch_idx;
+                *args.loss_sum += total;
+            }
+        }
+        return;
     }
+    int l = 0;
+    while (bx >= args.first[l + 1]) ++l;
+    const int at = bx - args.first[l];
+    if (l >= 3) {  // bias: lane y adds tiles y, y + 8, .. in order, then the 8 lane sums are added in order
+        const FinishBias &fb = args.bias[l - 3];
+        const int c = at * kTile + tx;
+        float sum = 0.f;
+        if (c < fb.cols)
+            for (int t = ty; t < args.tiles; t += kTileRows) sum += fb.part[(int64_t)t * fb.cols + c];
+        tile[ty][tx] = sum;
+        __syncthreads();
+        if (ty == 0 && c < fb.cols) {
+            float g = 0.f;
+            for (int y = 0; y < kTileRows; ++y) g += tile[y][tx];
+            args.grads[fb.off + c] = g;
+            const int64_t i = fb.off + c;
+            if (adam) adam_element(args.adam, i, g, args.adam.w[i], args.adam.m1[i], args.adam.m2[i], c1, c2);
+        }
+        return;
+    }
+    const FinishWeight &fw = args.w[l];
+    const int tiles_c = (fw.cols + kTile - 1) / kTile;
+    const int r0 = at / tiles_c * kTile, c0 = at % tiles_c * kTile;
+    const int c = c0 + tx;
+    const int64_t part = (int64_t)fw.rows * fw.ld;
+    constexpr int kRows = kTile / kTileRows;  // this thread's rows of the tile, loaded together
+    const bool in = c < fw.cols;
+    float g[kRows], w[kRows], m1[kRows], m2[kRows];
+    const float *p = fw.part + (int64_t)(r0 + ty) * fw.ld + c;
+    const int64_t i0 = fw.off + (int64_t)(r0 + ty) * fw.cols + c;
+#pragma unroll
+    for (int q = 0; q < kRows; ++q) {
+        const int64_t i = i0 + (int64_t)q * kTileRows * fw.cols;
+        g[q] = in ? p[(int64_t)q * kTileRows * fw.ld] : 0.f;
+        const bool load = in && adam;
+        w[q] = load ? args.adam.w[i] : 0.f;
+        m1[q] = load ? args.adam.m1[i] : 0.f;
+        m2[q] = load ? args.adam.m2[i] : 0.f;
+    }
+    if (in)
+#pragma unroll 4
+        for (int z = 1; z < args.splits; ++z)
+#pragma unroll
+            for (int q = 0; q < kRows; ++q) g[q] += p[z * part + (int64_t)q * kTileRows * fw.ld];
+#pragma unroll
+    for (int q = 0; q < kRows; ++q) {
+        float v = 0.f;
+        if (in) {
+            const int64_t i = i0 + (int64_t)q * kTileRows * fw.cols;
+            args.grads[i] = g[q];
+            if (adam) {
+                const __nv_bfloat16 b = __float2bfloat16_rn(adam_element(args.adam, i, g[q], w[q], m1[q], m2[q], c1, c2));
+                fw.b[(int64_t)(r0 + ty + q * kTileRows) * fw.ld + c] = b;
+                v = __bfloat162float(b);
+            }
+        }
+        tile[ty + q * kTileRows][tx] = v;
+    }
+    if (!adam || !fw.bt) return;
+    __syncthreads();
+    store_tile_t(tile, fw.bt, fw.rows, r0, c0, fw.rows, fw.cols);
 }
 
 __global__ void init_weights_kernel(float *w, int64_t n, float scale, uint64_t key) {
@@ -481,15 +478,29 @@ struct Mlp {
     // workspace for batches of up to cap_fwd rows (forward) / cap rows (backward)
     int64_t cap = 0;      // rows of the backward buffers
     int64_t cap_fwd = 0;  // rows of the forward buffers
-    DevBuf xb, h1, h2, pre1, pre2, y, dy, dyt, h2t, h1t, xbt, dh2, dp2, dp2t, dh1, dp1, dp1t, loss;
-    DevBuf gw1p;  // gradient of W1 in padded layout [h][dp]
-    DevBuf colws; // (cap / 32) x max(h, d_out) tile column sums
+    DevBuf xb, tb, h1, h2, slope1, slope2, dy, dyt, h2t, h1t, xbt, dp2, dp2t, dp1, dp1t, loss;
+    DevBuf wpart;  // the weight gradients' K parts (W1 padded to [h][dp])
+    DevBuf colws;  // (cap / 32) x (h + h + d_out) column sums over 32 rows
+    DevBuf lossp;  // (cap / 32) x (d_out / 32) sums of squared errors
 };
 
 namespace {
 
+int64_t wgrad_elems(const Mlp *mp) { return (int64_t)mp->h * mp->dp + (int64_t)mp->h * mp->h + (int64_t)mp->d_out * mp->h; }
+
+// dW3 = dY^T H2, dW2 = dZ2^T H1, dW1 = dZ1^T X (padded input columns give columns that are left
+// out), with `splits` parts each in mp->wpart.
+void wgrad_jobs(Mlp *mp, int splits, WgradJob *job) {
+    const int h = mp->h, dout = mp->d_out, dp = mp->dp;
+    float *w1 = mp->wpart.as<float>();
+    float *w2 = w1 + (int64_t)splits * h * dp, *w3 = w2 + (int64_t)splits * h * h;
+    job[0] = {mp->dp1t.p, mp->xbt.p, h, dp, w1};
+    job[1] = {mp->dp2t.p, mp->h1t.p, h, h, w2};
+    job[2] = {mp->dyt.p, mp->h2t.p, dout, h, w3};
+}
+
 // Workspace for batches of up to `rows` rows: the forward buffers, and with `train` also
-// those of the backward pass (the activations' transposes, pre-activations, gradients).
+// those of the backward pass (the batch's targets, the activations' transposes and slopes, gradients).
 int mlp_ensure(Mlp *mp, int64_t rows, bool train) {
     const int64_t r = (rows + 127) / 128 * 128;
     const size_t b2 = 2;
@@ -498,24 +509,27 @@ int mlp_ensure(Mlp *mp, int64_t rows, bool train) {
         CUMF_CUDA(mp->xb.alloc(r * dp * b2));
         CUMF_CUDA(mp->h1.alloc(r * h * b2));
         CUMF_CUDA(mp->h2.alloc(r * h * b2));
-        CUMF_CUDA(mp->y.alloc(r * dout * 4));
         mp->cap_fwd = r;
     }
     if (!train || rows <= mp->cap) return CUMF_OK;
-    CUMF_CUDA(mp->pre1.alloc(r * h * 4));
-    CUMF_CUDA(mp->pre2.alloc(r * h * 4));
+    CUMF_CUDA(mp->tb.alloc(r * dout * 4));
+    CUMF_CUDA(mp->slope1.alloc(r * h * 4));
+    CUMF_CUDA(mp->slope2.alloc(r * h * 4));
     CUMF_CUDA(mp->dy.alloc(r * dout * b2));
     CUMF_CUDA(mp->dyt.alloc(r * dout * b2));
     CUMF_CUDA(mp->h2t.alloc(r * h * b2));
     CUMF_CUDA(mp->h1t.alloc(r * h * b2));
     CUMF_CUDA(mp->xbt.alloc(r * dp * b2));
-    CUMF_CUDA(mp->dh2.alloc(r * h * 4));
     CUMF_CUDA(mp->dp2.alloc(r * h * b2));
     CUMF_CUDA(mp->dp2t.alloc(r * h * b2));
-    CUMF_CUDA(mp->dh1.alloc(r * h * 4));
     CUMF_CUDA(mp->dp1.alloc(r * h * b2));
     CUMF_CUDA(mp->dp1t.alloc(r * h * b2));
-    CUMF_CUDA(mp->colws.alloc((r / kTile) * (h > dout ? h : dout) * 4));
+    CUMF_CUDA(mp->colws.alloc((r / kTile) * (2 * h + dout) * 4));
+    CUMF_CUDA(mp->lossp.alloc((r / kTile) * (dout / kTile) * sizeof(double)));
+    // The parts of the longest K that this workspace serves: fewer rows are split no further.
+    WgradJob jobs[kWgradJobs];
+    wgrad_jobs(mp, 1, jobs);
+    CUMF_CUDA(mp->wpart.alloc((size_t)wgrad_splits(jobs, r) * wgrad_elems(mp) * 4));
     mp->cap = r;
     return CUMF_OK;
 }
@@ -527,12 +541,13 @@ dim3 tiles_of(int64_t rows, int cols) { return dim3((unsigned)((rows + kTile - 1
 ConvertJob convert_job(const float *S, int cols, const int32_t *perm, const int *batch_idx, int64_t batch, int valid,
                        int rp, int ldd, void *D, void *Dt) {
     return ConvertJob{S, cols, perm, batch_idx, batch, valid, rp, ldd, static_cast<__nv_bfloat16 *>(D),
-                      static_cast<__nv_bfloat16 *>(Dt)};
+                      static_cast<__nv_bfloat16 *>(Dt), nullptr};
 }
 
 // n (1..3) conversions in one launch.
-cudaError_t convert(const ConvertJob *job, int n, cudaStream_t s) {
+cudaError_t convert(const ConvertJob *job, int n, cudaStream_t s, int64_t *step = nullptr) {
     ConvertJobs jobs{};
+    jobs.step = step;
     unsigned gx = 1, gy = 1;
     for (int i = 0; i < n; ++i) {
         jobs.job[i] = job[i];
@@ -541,18 +556,6 @@ cudaError_t convert(const ConvertJob *job, int n, cudaStream_t s) {
         gy = g.y > gy ? g.y : gy;
     }
     convert_t_kernel<<<dim3(gx, gy, n), kTileBlock, 0, s>>>(jobs);
-    return cudaGetLastError();
-}
-
-cudaError_t transpose(const void *D, int rows, int cols, void *Dt, cudaStream_t s) {
-    transpose_t_kernel<<<tiles_of(rows, cols), kTileBlock, 0, s>>>(static_cast<const __nv_bfloat16 *>(D), rows, cols,
-                                                                   static_cast<__nv_bfloat16 *>(Dt));
-    return cudaGetLastError();
-}
-
-cudaError_t colsum_finish(Mlp *mp, int64_t rp, int cols, float *out, cudaStream_t s) {
-    colsum_finish_kernel<<<(cols + kTile - 1) / kTile, kTileBlock, 0, s>>>(mp->colws.as<float>(), (int)(rp / kTile),
-                                                                            cols, out);
     return cudaGetLastError();
 }
 
@@ -568,65 +571,99 @@ int mlp_refresh(Mlp *mp, cudaStream_t s) {
     return CUMF_OK;
 }
 
-// Forward over rows [0, rows) of X (fp32, rows x d_in; with perm, row r is X[perm[*batch_idx *
-// batch + r]]); Y (fp32 rows x d_out) in Y, or with its padding rows in mp->y.  train: also X's bf16 transpose and the
-// pre-activations, which the backward pass uses.
-int mlp_forward_ws(Mlp *mp, const float *X, int64_t rows, cudaStream_t s, bool train, const int32_t *perm = nullptr,
-                   const int *batch_idx = nullptr, int64_t batch = 0, float *Y = nullptr) {
-    if (int rc = mlp_ensure(mp, rows, train)) return rc;
+// Y (fp32 rows x d_out) of rows [0, rows) of X (fp32 rows x d_in).
+int mlp_forward_ws(Mlp *mp, const float *X, int64_t rows, float *Y, cudaStream_t s) {
+    if (int rc = mlp_ensure(mp, rows, false)) return rc;
     const float *P = mp->params.as<float>();
     const int h = mp->h;
     const int64_t rp = (rows + 127) / 128 * 128;  // padding rows are zero
-    const ConvertJob job = convert_job(X, mp->d_in, perm, batch_idx, batch, (int)rows, (int)rp, mp->dp, mp->xb.p,
-                                       train ? mp->xbt.p : nullptr);
+    const ConvertJob job = convert_job(X, mp->d_in, nullptr, nullptr, 0, (int)rows, (int)rp, mp->dp, mp->xb.p, nullptr);
     CUMF_CUDA(convert(&job, 1, s));
     int *st = mp->status.as<int>();
-    CUMF_CUDA(launch_tc_gemm(mp->xb.p, mp->w1b.p, (int)rp, h, mp->dp, P + mp->off_b1, 1, mp->h1.p, 0, h,
-                             train ? mp->pre1.as<float>() : nullptr, st, s));
-    CUMF_CUDA(launch_tc_gemm(mp->h1.p, mp->w2b.p, (int)rp, h, h, P + mp->off_b2, 1, mp->h2.p, 0, h,
-                             train ? mp->pre2.as<float>() : nullptr, st, s));
-    CUMF_CUDA(launch_tc_gemm(mp->h2.p, mp->w3b.p, (int)(Y ? rows : rp), mp->d_out, h, P + mp->off_b3, 0,
-                             Y ? Y : mp->y.as<float>(), 1, mp->d_out, nullptr, st, s));
+    CUMF_CUDA(launch_tc_gemm(mp->xb.p, mp->w1b.p, (int)rp, h, mp->dp, P + mp->off_b1, 1, mp->h1.p, 0, h, nullptr, st, s));
+    CUMF_CUDA(launch_tc_gemm(mp->h1.p, mp->w2b.p, (int)rp, h, h, P + mp->off_b2, 1, mp->h2.p, 0, h, nullptr, st, s));
+    CUMF_CUDA(launch_tc_gemm(mp->h2.p, mp->w3b.p, (int)rows, mp->d_out, h, P + mp->off_b3, 0, Y, 1, mp->d_out, nullptr,
+                             st, s));
     return CUMF_OK;
 }
 
-// Loss and gradients (into mp->grads) for rows [0, rows) with targets T (fp32 rows x d_out,
-// through perm as in mlp_forward_ws), after mlp_forward_ws on the same rows.
-int mlp_backward_ws(Mlp *mp, const float *T, int64_t rows, cudaStream_t s, const int32_t *perm = nullptr,
-                    const int *batch_idx = nullptr, int64_t batch = 0) {
+// The batch of a step: row r is X[perm[*batch_idx * batch + r]] (perm NULL: X[r]), T likewise.
+struct Batch {
+    const float *X, *T;
+    int64_t rows;
+    const int32_t *perm;
+    int *batch_idx;
+    int64_t batch;
+};
+
+// Loss (mp->loss) and gradients (mp->grads) of a batch; with `adam` (its step count advanced
+// first), also the update, the next batch's index and the loss added to *loss_sum.
+int mlp_step_ws(Mlp *mp, const Batch &bt, cudaStream_t s, const Adam &adam = Adam{}, int64_t *step = nullptr,
+                double *loss_sum = nullptr) {
+    if (int rc = mlp_ensure(mp, bt.rows, true)) return rc;
+    const float *P = mp->params.as<float>();
     const int h = mp->h, dout = mp->d_out, dp = mp->dp;
-    const int64_t rp = (rows + 127) / 128 * 128;
-    float *G = mp->grads.as<float>();
-    float *part = mp->colws.as<float>();
+    const int rows = (int)bt.rows, rp = (int)((bt.rows + 127) / 128 * 128);  // padding rows are zero
+    const int tiles = rp / kTile;
+    float *col1 = mp->colws.as<float>(), *col2 = col1 + (int64_t)tiles * h, *col3 = col2 + (int64_t)tiles * h;
     int *st = mp->status.as<int>();
-    CUMF_CUDA(cudaMemsetAsync(mp->loss.p, 0, sizeof(double), s));
-    // layer 3: dY (and dY^T, db3), dW3 = dY^T H2, dH2 = dY W3
-    mse_grad_t_kernel<<<tiles_of(rp, dout), kTileBlock, 0, s>>>(
-        mp->y.as<float>(), T, perm, batch_idx, batch, (int)rp, (int)rows, dout, 1.f / (float)rows,
-        mp->dy.as<__nv_bfloat16>(), mp->dyt.as<__nv_bfloat16>(), part, mp->loss.as<double>());
+    // X's two copies; the targets' rows too where they are gathered (with the many blocks of this
+    // launch, not behind two dependent loads in each block of the loss)
+    ConvertJob job[2] = {
+        convert_job(bt.X, mp->d_in, bt.perm, bt.batch_idx, bt.batch, rows, rp, dp, mp->xb.p, mp->xbt.p),
+        convert_job(bt.T, dout, bt.perm, bt.batch_idx, bt.batch, rows, rp, dout, nullptr, nullptr)};
+    job[1].F = mp->tb.as<float>();
+    CUMF_CUDA(convert(job, bt.perm ? 2 : 1, s, step));
+    auto ep = [&](DevBuf &out, DevBuf &out_t) {
+        TrainEpilogue e{};
+        e.out = out.as<__nv_bfloat16>();
+        e.out_t = out_t.as<__nv_bfloat16>();
+        e.valid = rows;
+        return e;
+    };
+    TrainEpilogue e1 = ep(mp->h1, mp->h1t), e2 = ep(mp->h2, mp->h2t), e3 = ep(mp->dy, mp->dyt);
+    TrainEpilogue g2 = ep(mp->dp2, mp->dp2t), g1 = ep(mp->dp1, mp->dp1t);
+    e1.bias = P + mp->off_b1, e1.slope = mp->slope1.as<float>();
+    e2.bias = P + mp->off_b2, e2.slope = mp->slope2.as<float>();
+    e3.bias = P + mp->off_b3, e3.T = bt.perm ? mp->tb.as<float>() : bt.T;
+    e3.scale = 1.f / (float)rows, e3.colsum = col3, e3.loss = mp->lossp.as<double>();
+    g2.slope = e2.slope, g2.colsum = col2;
+    g1.slope = e1.slope, g1.colsum = col1;
+    // H1, H2, dY, then dZ2 = dY W3 * slope2, dZ1 = dZ2 W2 * slope1, then the weight gradients
+    CUMF_CUDA(launch_train_gemm(kTrainForward, mp->xb.p, mp->w1b.p, rp, h, dp, e1, st, s));
+    CUMF_CUDA(launch_train_gemm(kTrainForward, mp->h1.p, mp->w2b.p, rp, h, h, e2, st, s));
+    CUMF_CUDA(launch_train_gemm(kTrainLoss, mp->h2.p, mp->w3b.p, rp, dout, h, e3, st, s));
+    CUMF_CUDA(launch_train_gemm(kTrainBack, mp->dy.p, mp->w3t.p, rp, h, dout, g2, st, s));
+    CUMF_CUDA(launch_train_gemm(kTrainBack, mp->dp2.p, mp->w2t.p, rp, h, h, g1, st, s));
+    WgradJob jobs[kWgradJobs];
+    wgrad_jobs(mp, 1, jobs);
+    const int splits = wgrad_splits(jobs, rp);
+    wgrad_jobs(mp, splits, jobs);
+    CUMF_CUDA(launch_wgrad(jobs, rp, splits, st, s));
+
+    FinishArgs f{};
+    auto bf = [](DevBuf &b) { return b.as<__nv_bfloat16>(); };
+    f.w[0] = {jobs[0].out, mp->off_w1, h, mp->d_in, dp, bf(mp->w1b), nullptr};
+    f.w[1] = {jobs[1].out, mp->off_w2, h, h, h, bf(mp->w2b), bf(mp->w2t)};
+    f.w[2] = {jobs[2].out, mp->off_w3, dout, h, h, bf(mp->w3b), bf(mp->w3t)};
+    f.bias[0] = {col1, mp->off_b1, h};
+    f.bias[1] = {col2, mp->off_b2, h};
+    f.bias[2] = {col3, mp->off_b3, dout};
+    for (int l = 0; l < 3; ++l) {
+        f.first[l + 1] = f.first[l] + f.w[l].rows / kTile * ((f.w[l].cols + kTile - 1) / kTile);
+    }
+    for (int l = 0; l < 3; ++l) f.first[l + 4] = f.first[l + 3] + f.bias[l].cols / kTile;
+    f.splits = splits;
+    f.tiles = tiles;
+    f.grads = mp->grads.as<float>();
+    f.adam = adam;
+    f.loss_part = mp->lossp.as<double>();
+    f.loss_parts = tiles * (dout / kTile);
+    f.loss = mp->loss.as<double>();
+    f.loss_sum = loss_sum;
+    f.batch_idx = loss_sum ? bt.batch_idx : nullptr;
+    finish_step_kernel<<<f.first[6] + 1, kTileBlock, 0, s>>>(f);
     CUMF_CUDA(cudaGetLastError());
-    CUMF_CUDA(colsum_finish(mp, rp, dout, G + mp->off_b3, s));
-    CUMF_CUDA(transpose(mp->h2.p, (int)rp, h, mp->h2t.p, s));
-    CUMF_CUDA(launch_tc_gemm(mp->dyt.p, mp->h2t.p, dout, h, (int)rp, nullptr, 0, G + mp->off_w3, 1, h, nullptr, st, s));
-    CUMF_CUDA(launch_tc_gemm(mp->dy.p, mp->w3t.p, (int)rp, h, dout, nullptr, 0, mp->dh2.p, 1, h, nullptr, st, s));
-    // layer 2
-    gelu_back_t_kernel<<<tiles_of(rp, h), kTileBlock, 0, s>>>(mp->dh2.as<float>(), mp->pre2.as<float>(), (int)rp,
-                                                              (int)rows, h, mp->dp2.as<__nv_bfloat16>(),
-                                                              mp->dp2t.as<__nv_bfloat16>(), part);
-    CUMF_CUDA(cudaGetLastError());
-    CUMF_CUDA(colsum_finish(mp, rp, h, G + mp->off_b2, s));
-    CUMF_CUDA(transpose(mp->h1.p, (int)rp, h, mp->h1t.p, s));
-    CUMF_CUDA(launch_tc_gemm(mp->dp2t.p, mp->h1t.p, h, h, (int)rp, nullptr, 0, G + mp->off_w2, 1, h, nullptr, st, s));
-    CUMF_CUDA(launch_tc_gemm(mp->dp2.p, mp->w2t.p, (int)rp, h, h, nullptr, 0, mp->dh1.p, 1, h, nullptr, st, s));
-    // layer 1 (padded input columns give zero gradient columns, dropped on copy)
-    gelu_back_t_kernel<<<tiles_of(rp, h), kTileBlock, 0, s>>>(mp->dh1.as<float>(), mp->pre1.as<float>(), (int)rp,
-                                                              (int)rows, h, mp->dp1.as<__nv_bfloat16>(),
-                                                              mp->dp1t.as<__nv_bfloat16>(), part);
-    CUMF_CUDA(cudaGetLastError());
-    CUMF_CUDA(colsum_finish(mp, rp, h, G + mp->off_b1, s));
-    CUMF_CUDA(launch_tc_gemm(mp->dp1t.p, mp->xbt.p, h, dp, (int)rp, nullptr, 0, mp->gw1p.p, 1, dp, nullptr, st, s));
-    CUMF_CUDA(cudaMemcpy2DAsync(G + mp->off_w1, mp->d_in * sizeof(float), mp->gw1p.p, dp * sizeof(float),
-                                mp->d_in * sizeof(float), h, cudaMemcpyDeviceToDevice, s));
     return CUMF_OK;
 }
 
@@ -672,7 +709,6 @@ int cumf_mlp_create(int d_in, int hidden, int d_out, uint64_t seed, void **out) 
     if (cudaError_t e = mp->w3b.alloc((size_t)d_out * hidden * 2)) return cleanup(cuda_fail(e, "mlp w3"));
     if (cudaError_t e = mp->w2t.alloc((size_t)hidden * hidden * 2)) return cleanup(cuda_fail(e, "mlp w2t"));
     if (cudaError_t e = mp->w3t.alloc((size_t)d_out * hidden * 2)) return cleanup(cuda_fail(e, "mlp w3t"));
-    if (cudaError_t e = mp->gw1p.alloc((size_t)hidden * mp->dp * 4)) return cleanup(cuda_fail(e, "mlp gw1"));
     if (cudaError_t e = mp->status.alloc(sizeof(int))) return cleanup(cuda_fail(e, "mlp status"));
     if (cudaError_t e = mp->loss.alloc(sizeof(double))) return cleanup(cuda_fail(e, "mlp loss"));
     cudaMemset(mp->status.p, 0, sizeof(int));
@@ -726,8 +762,7 @@ int cumf_mlp_forward(void *mlp, const float *d_X, int64_t rows, float *d_Y, void
     const int64_t chunk = 1 << 16;
     for (int64_t r0 = 0; r0 < rows; r0 += chunk) {
         const int64_t r = std::min(chunk, rows - r0);
-        if (int rc = mlp_forward_ws(mp, d_X + r0 * mp->d_in, r, s, false, nullptr, nullptr, 0, d_Y + r0 * mp->d_out))
-            return rc;
+        if (int rc = mlp_forward_ws(mp, d_X + r0 * mp->d_in, r, d_Y + r0 * mp->d_out, s)) return rc;
     }
     return mlp_check_status(mp, s);
 }
@@ -736,8 +771,7 @@ int cumf_mlp_loss_grad(void *mlp, const float *d_X, const float *d_T, int64_t ro
     Mlp *mp = static_cast<Mlp *>(mlp);
     if (!mp || !d_X || !d_T || rows <= 0) return fail(CUMF_ERR_ARG, "mlp_loss_grad: bad arguments");
     cudaStream_t s = (cudaStream_t)stream;
-    if (int rc = mlp_forward_ws(mp, d_X, rows, s, true)) return rc;
-    if (int rc = mlp_backward_ws(mp, d_T, rows, s)) return rc;
+    if (int rc = mlp_step_ws(mp, Batch{d_X, d_T, rows, nullptr, nullptr, 0}, s)) return rc;
     double l = 0;
     CUMF_CUDA(cudaMemcpyAsync(&l, mp->loss.p, sizeof(double), cudaMemcpyDeviceToHost, s));
     if (int rc = mlp_check_status(mp, s)) return rc;
@@ -804,16 +838,9 @@ int cumf_mlp_train(void *mlp, const float *d_X, const float *d_T, int64_t rows, 
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     // One training step of r rows at the batch the device index names.
     auto enqueue_step = [&](int64_t r) -> int {
-        const int32_t *perm = perm_d.as<int32_t>();
-        if (int rc = mlp_forward_ws(mp, d_X, r, ws, true, perm, &st->batch_idx, batch)) return rc;
-        if (int rc = mlp_backward_ws(mp, d_T, r, ws, perm, &st->batch_idx, batch)) return rc;
-        adam_kernel<<<grid_of(mp->count), kT, 0, ws>>>(mp->params.as<float>(), mp->grads.as<float>(),
-                                                       mp->m1.as<float>(), mp->m2.as<float>(), mp->count, lr, b1, b2,
-                                                       eps, &st->step);
-        if (int rc = mlp_refresh(mp, ws)) return rc;
-        step_end_kernel<<<1, 1, 0, ws>>>(&st->step, &st->batch_idx, mp->loss.as<double>(), &st->loss_sum);
-        CUMF_CUDA(cudaGetLastError());
-        return CUMF_OK;
+        const Adam adam = {mp->params.as<float>(), mp->m1.as<float>(), mp->m2.as<float>(), lr, b1, b2, eps, &st->step};
+        return mlp_step_ws(mp, Batch{d_X, d_T, r, perm_d.as<int32_t>(), &st->batch_idx, batch}, ws, adam, &st->step,
+                           &st->loss_sum);
     };
     // Capture the full-batch step and the last, shorter one; replay them every epoch.
     auto capture = [&](int64_t r, cudaGraphExec_t *exec) -> int {

@@ -3,7 +3,8 @@
 //   C[M x N] = act(A[M x K] * B[N x K]^T + bias[N])       (A, B bf16 row-major; fp32 accumulate)
 //
 // Used by the warm-start MLP (forward: activations x W^T; backward: dX = dY W and
-// dW = dY^T X, given as TN products on transposed copies).  One CTA of 256 threads computes a
+// dW = dY^T X, given as TN products on transposed copies; a training step's products have their
+// own epilogues, tc_train_kernel and tc_wgrad_kernel below).  One CTA of 256 threads computes a
 // 128 x BN tile (BN = 128 or 256):
 //   - thread 0 is the TMA producer: operand tiles of 64 K-elements (128-byte rows) arrive by
 //     cp.async.bulk.tensor.2d with the 128-byte swizzle into a ring of shared memory (2 stages
@@ -18,9 +19,8 @@
 //     columns at a time), add the bias, apply the activation, and pass each 32 x 32 block
 //     through shared memory (the idle operand ring) so that the global stores are whole
 //     128-byte lines;
-//   - when the output has too few tiles to fill the GPU and K is long (the weight gradients),
-//     K is split over grid.z and the partial tiles are added into a zeroed fp32 output with
-//     vector atomics.
+//   - when the output has too few tiles to fill the GPU and K is long, K is split over grid.z
+//     and the partial tiles are added into a zeroed fp32 output with vector atomics.
 // Every mbarrier wait is bounded; on timeout the kernel records CUMF_ERR_TIMEOUT, stops
 // issuing work, waits (bounded) for what it issued and releases its tensor memory.
 #include <cuda.h>
@@ -34,6 +34,7 @@
 
 #include "cumf_sgd.h"
 #include "internal.h"
+#include "tc_gemm.h"
 
 namespace cumf {
 
@@ -213,42 +214,44 @@ struct TmaSmem {
     static constexpr int TOTAL = 1024 + kStages * STAGE + 256;  // alignment slack + barriers
 };
 
+// One CTA's 128 x BN accumulator: the operand ring and barriers in shared memory, and the tensor
+// memory.  Every thread of the CTA calls setup_tile, tile_product and, after the epilogue,
+// release_tile.
 template <int BN, int kStages>
-__global__ void __launch_bounds__(kTcThreads, kStages == 2 ? 2 : 1)
-tc_gemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, int M,
-                   int N, int K, const float *__restrict__ bias, int act, void *out, int out_f32, int ldo,
-                   float *pre_out, int *status, int splits, int no_copies) {
-    using S = TmaSmem<BN, kStages>;
-    extern __shared__ unsigned char smem_raw[];
+struct Tile {
+    unsigned char *ring;
+    uint64_t *full, *empty, *done;
+    int *abort_flag, *issued_slot;
+    uint32_t tmem;
+};
+
+template <int BN, int kStages>
+__device__ __forceinline__ Tile<BN, kStages> setup_tile(unsigned char *smem_raw, const CUtensorMap &map_a,
+                                                        const CUtensorMap &map_b) {
+    Tile<BN, kStages> t;
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;  // swizzle atoms need 1024-byte alignment
-    unsigned char *bar_area = smem_raw + (base - raw) + kStages * S::STAGE;
-    uint64_t *full = reinterpret_cast<uint64_t *>(bar_area);
-    uint64_t *empty = full + kStages;
-    uint64_t *done = empty + kStages;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + 1);
-    int *abort_flag = reinterpret_cast<int *>(tmem_slot + 1);
-    int *issued_slot = abort_flag + 1;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int m0 = blockIdx.x * kTcBM, n0 = blockIdx.y * BN;
-    const int KT_all = (K + kTcBK - 1) / kTcBK;
-    const int kt0 = (int)((long long)KT_all * blockIdx.z / splits);
-    const int kt1 = (int)((long long)KT_all * (blockIdx.z + 1) / splits);
-    const int KT = kt1 - kt0;
+    t.ring = smem_raw + (base - raw);
+    t.full = reinterpret_cast<uint64_t *>(t.ring + kStages * TmaSmem<BN, kStages>::STAGE);
+    t.empty = t.full + kStages;
+    t.done = t.empty + kStages;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(t.done + 1);
+    t.abort_flag = reinterpret_cast<int *>(tmem_slot + 1);
+    t.issued_slot = t.abort_flag + 1;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < kStages; ++i) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&full[i])));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&empty[i])));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&t.full[i])));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&t.empty[i])));
         }
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(done)));
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(t.done)));
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-        *abort_flag = 0;
-        *issued_slot = 0;
+        *t.abort_flag = 0;
+        *t.issued_slot = 0;
         asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(&map_a)) : "memory");
         asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(&map_b)) : "memory");
     }
-    if (warp == 0) {
+    if (threadIdx.x < 32) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tmem_slot)),
                      "r"(BN));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
@@ -256,7 +259,20 @@ tc_gemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const uint32_t tmem = *tmem_slot;
+    t.tmem = *tmem_slot;
+    return t;
+}
+
+// The product over the K stages kt0 .. kt0 + KT: thread 0 streaming, thread 32 issuing, every
+// thread waiting.  Returns whether the accumulator is valid; the operand ring is idle then.
+template <int BN, int kStages>
+__device__ __forceinline__ bool tile_product(const Tile<BN, kStages> &t, const CUtensorMap &map_a,
+                                             const CUtensorMap &map_b, int m0, int n0, int kt0, int KT, int *status,
+                                             int no_copies) {
+    using S = TmaSmem<BN, kStages>;
+    uint64_t *full = t.full, *empty = t.empty, *done = t.done;
+    int *abort_flag = t.abort_flag, *issued_slot = t.issued_slot;
+    const uint32_t base = smem_u32(t.ring), tmem = t.tmem;
 
     if (threadIdx.x == 0 && KT > 0 && !no_copies) {  // TMA producer (no_copies: the wait self-test)
         for (int i = 0; i < KT; ++i) {
@@ -314,35 +330,265 @@ tc_gemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             }
             mbar_wait(smem_u32(done), 0);
         }
-    } else if (KT > 0) {
-        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        // Warp w reads tensor-memory lanes 32 (w % 4).. (its rows) and half w / 4 of the
-        // columns.  The operand ring is idle now and holds each warp's staging block.
-        float *stg = reinterpret_cast<float *>(smem_raw + (base - raw)) + warp * (32 * kStgStride);
-        const int quarter = warp & 3, half = warp >> 2;
-        const int r0 = m0 + quarter * 32;
+        return false;
+    }
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    return KT > 0;
+}
+
+template <int BN>
+__device__ __forceinline__ void release_tile(uint32_t tmem) {
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(BN));
+    }
+}
+
+// The accumulator's 32 columns c0.. of this warp's 32 tensor-memory lanes (32 (warp % 4)..).
+__device__ __forceinline__ void load_acc(uint32_t (&r)[32], uint32_t tmem, int c0) {
+    const uint32_t taddr = tmem + ((uint32_t)((threadIdx.x >> 5 & 3) * 32) << 16) + (uint32_t)c0;
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
+        "%13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, "
+        "[%32];\n"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
+          "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]),
+          "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]),
+          "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+}
+
+template <int BN, int kStages>
+__global__ void __launch_bounds__(kTcThreads, kStages == 2 ? 2 : 1)
+tc_gemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, int M,
+                   int N, int K, const float *__restrict__ bias, int act, void *out, int out_f32, int ldo,
+                   float *pre_out, int *status, int splits, int no_copies) {
+    extern __shared__ unsigned char smem_raw[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int m0 = blockIdx.x * kTcBM, n0 = blockIdx.y * BN;
+    const int KT_all = (K + kTcBK - 1) / kTcBK;
+    const int kt0 = (int)((long long)KT_all * blockIdx.z / splits);
+    const int kt1 = (int)((long long)KT_all * (blockIdx.z + 1) / splits);
+    const Tile<BN, kStages> t = setup_tile<BN, kStages>(smem_raw, map_a, map_b);
+    if (tile_product(t, map_a, map_b, m0, n0, kt0, kt1 - kt0, status, no_copies)) {
+        // Warp w: half w / 4 of the columns; the idle ring holds each warp's staging block.
+        float *stg = reinterpret_cast<float *>(t.ring) + warp * (32 * kStgStride);
+        const int half = warp >> 2, r0 = m0 + (warp & 3) * 32;
         for (int c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2) && n0 + c0 < N; c0 += 32) {
             uint32_t r[32];
-            const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0;
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
-                "%13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, "
-                "[%32];\n"
-                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                  "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-                  "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]),
-                  "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]),
-                  "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-                : "r"(taddr));
-            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+            load_acc(r, t.tmem, c0);
             epilogue_chunk(stg, r, r0, n0 + c0, M, N, bias, act, out, out_f32, ldo, pre_out, splits > 1, lane);
         }
     }
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
-    if (warp == 0) {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(BN));
+    release_tile<BN>(t.tmem);
+}
+
+// ---- products of a training step ----------------------------------------------------------
+
+// gelu(x) as above, and its derivative: they share the tanh, which is most of either.
+__device__ __forceinline__ float gelu_slope(float x, float &slope) {
+    const float c = 0.7978845608028654f;
+    const float t = tanhf(c * (x + 0.044715f * x * x * x));
+    slope = 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * c * (1.f + 3.f * 0.044715f * x * x);
+    return 0.5f * x * (1.0f + t);
+}
+
+// a + b = s + err exactly (Knuth's two-sum).
+__device__ __forceinline__ float two_sum(float a, float b, float &err) {
+    const float s = __fadd_rn(a, b), z = __fsub_rn(s, a);
+    err = __fadd_rn(__fsub_rn(a, __fsub_rn(s, z)), __fsub_rn(b, z));
+    return s;
+}
+
+// The sum of d[j]^2 as a double.  FP64 arithmetic is some sixty times slower than FP32 here, so
+// the exact squares (product and its fma remainder) are added in three floats whose roundings are
+// kept (72 bits); values whose squares or remainders would leave FP32's range go through double.
+__device__ __forceinline__ double sum_squares(const float (&d)[32]) {
+    float top = 0.f;
+#pragma unroll
+    for (int j = 0; j < 32; ++j) top = fmaxf(top, fabsf(d[j]));
+    if (top < 1.152921504606847e18f && (top > 9.313225746154785e-10f || top == 0.f)) {  // 2^60, 2^-30
+        float hi = 0.f, mid = 0.f, lo = 0.f;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            const float p = __fmul_rn(d[j], d[j]), e = __fmaf_rn(d[j], d[j], -p);
+            float a, b, c;
+            hi = two_sum(hi, p, a);
+            mid = two_sum(mid, a, b);
+            mid = two_sum(mid, e, c);
+            lo = __fadd_rn(lo, __fadd_rn(b, c));
+        }
+        return (double)hi + ((double)mid + (double)lo);
     }
+    double sum = 0;
+    for (int j = 0; j < 32; ++j) sum += (double)d[j] * d[j];
+    return sum;
+}
+
+// Two bf16 values of exactly representable floats.
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
+
+// A warp's 32 x 32 block (lane = row) of bf16 values, to out (ldo columns) and out_t (ldt rows);
+// with colsum, the block's column sums: rows y, y + 8, y + 16, y + 24 for each y < 8, then these
+// eight sums, in order.
+__device__ __forceinline__ void write_both(float *stg, const float (&v)[32], int r0, int col0, __nv_bfloat16 *out,
+                                           int ldo, __nv_bfloat16 *out_t, int ldt, float *colsum, int lane) {
+    stage_f32(stg, v, lane);
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {  // four lanes per row, 16 bytes each
+        const int row = it * 8 + (lane >> 2), c = (lane & 3) * 8;
+        const float4 a = *reinterpret_cast<const float4 *>(stg + row * kStgStride + c);
+        const float4 b = *reinterpret_cast<const float4 *>(stg + row * kStgStride + c + 4);
+        *reinterpret_cast<uint4 *>(out + (size_t)(r0 + row) * ldo + col0 + c) =
+            make_uint4(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w), pack_bf16(b.x, b.y), pack_bf16(b.z, b.w));
+    }
+    float x[32];  // lane = column
+#pragma unroll
+    for (int i = 0; i < 32; ++i) x[i] = stg[i * kStgStride + lane];
+    uint4 *t = reinterpret_cast<uint4 *>(out_t + (size_t)(col0 + lane) * ldt + r0);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        t[q] = make_uint4(pack_bf16(x[8 * q], x[8 * q + 1]), pack_bf16(x[8 * q + 2], x[8 * q + 3]),
+                          pack_bf16(x[8 * q + 4], x[8 * q + 5]), pack_bf16(x[8 * q + 6], x[8 * q + 7]));
+    if (colsum) {
+        float total = 0.f;
+#pragma unroll
+        for (int y = 0; y < 8; ++y) total += ((x[y] + x[y + 8]) + x[y + 16]) + x[y + 24];
+        colsum[(size_t)(r0 >> 5) * ldo + col0 + lane] = total;
+    }
+}
+
+// A 128 x BN tile by 4 BN threads, so that each warp's epilogue is one 32 x 32 block: the
+// activation's arithmetic and the stores' latency, not the product (K of a few stages), are what
+// these kernels take.  Fused, because every pass over a 4096 x 512 batch between the products
+// (transposes, gelu', column sums, loss) was a launch of 2 to 8 us: a training step of 4096 rows
+// (131 -> 512 -> 512 -> 128) took 127 us of device time in 25 launches, 68 in 8.
+// What the epilogue reads (slopes, targets) is fetched before the product's waits.
+template <int BN, int kStages, int MODE>
+__global__ void __launch_bounds__(4 * BN, BN == 128 ? 1 : 2)
+tc_train_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, int M, int N,
+                int K, const __grid_constant__ TrainEpilogue ep, int *status) {
+    static_assert(4 * BN / 32 * 32 * kStgStride * 4 <= kStages * TmaSmem<BN, kStages>::STAGE, "staging fits the ring");
+    extern __shared__ unsigned char smem_raw[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n0 = blockIdx.y * BN, c0 = (warp >> 2) * 32;
+    const int r0 = blockIdx.x * kTcBM + (warp & 3) * 32, col0 = n0 + c0;
+    const bool mine = col0 < N;
+    const Tile<BN, kStages> t = setup_tile<BN, kStages>(smem_raw, map_a, map_b);
+    float4 in[8];  // the 32 x 32 block of slope or T: lane's rows 4 it + lane / 8, columns 4 (lane % 8)
+    if (MODE != kTrainForward) {
+        const float *src = MODE == kTrainLoss ? ep.T : ep.slope;
+        const bool vec = (reinterpret_cast<uintptr_t>(src) & 15) == 0;  // N is a multiple of 32
+#pragma unroll
+        for (int it = 0; it < 8; ++it) {
+            const int r = r0 + it * 4 + (lane >> 3);
+            in[it] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (mine && r < ep.valid) {
+                const float *p = src + (int64_t)r * N + col0 + (lane & 7) * 4;
+                in[it] = vec ? *reinterpret_cast<const float4 *>(p) : make_float4(p[0], p[1], p[2], p[3]);
+            }
+        }
+    }
+    const bool ok = tile_product(t, map_a, map_b, blockIdx.x * kTcBM, n0, 0, (K + kTcBK - 1) / kTcBK, status, 0);
+    if (ok && mine) {
+        float *stg = reinterpret_cast<float *>(t.ring) + warp * (32 * kStgStride);
+        uint32_t r[32];
+        float v[32];
+        load_acc(r, t.tmem, c0);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+        if (MODE != kTrainBack) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const float4 b = __ldg(reinterpret_cast<const float4 *>(ep.bias + col0) + q);
+                v[4 * q] += b.x, v[4 * q + 1] += b.y, v[4 * q + 2] += b.z, v[4 * q + 3] += b.w;
+            }
+        }
+        if (MODE == kTrainForward) {
+            float slope[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = gelu_slope(v[j], slope[j]);
+            stage_f32(stg, slope, lane);
+            write_f32(stg, ep.slope, r0, col0, M, N, N, true, false, lane);
+        } else {
+            float w[32];  // the staged block's row `lane`
+#pragma unroll
+            for (int it = 0; it < 8; ++it)
+                *reinterpret_cast<float4 *>(stg + (it * 4 + (lane >> 3)) * kStgStride + (lane & 7) * 4) = in[it];
+            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const float4 x = *reinterpret_cast<const float4 *>(stg + lane * kStgStride + 4 * q);
+                w[4 * q] = x.x, w[4 * q + 1] = x.y, w[4 * q + 2] = x.z, w[4 * q + 3] = x.w;
+            }
+            const bool valid = r0 + lane < ep.valid;
+            if (MODE == kTrainLoss) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = valid ? v[j] - w[j] : 0.f;
+                double sum = sum_squares(v);
+#pragma unroll
+                for (int o = 16; o >= 1; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                if (lane == 0) ep.loss[(size_t)(r0 >> 5) * (N >> 5) + (col0 >> 5)] = sum;
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = 2.f * v[j] * ep.scale;
+            } else {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = valid ? v[j] * w[j] : 0.f;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = __bfloat162float(__float2bfloat16_rn(v[j]));
+        write_both(stg, v, r0, col0, ep.out, N, ep.out_t, M, MODE == kTrainForward ? nullptr : ep.colsum, lane);
+    }
+    release_tile<BN>(t.tmem);
+}
+
+// The three weight gradients of a step: 128 x 128 tiles of all of them, K split so that they make
+// one wave, each part stored by itself.  One launch, since each alone leaves most SMs idle or
+// waits for its own first loads; the parts are added by the kernel that applies them, in order, so
+// that neither a zeroed output nor atomics are needed and a step gives the same bits every run.
+struct WgradArgs {
+    CUtensorMap a[kWgradJobs], b[kWgradJobs];
+    int M[kWgradJobs], N[kWgradJobs], first[kWgradJobs];  // first: a job's first block
+    float *out[kWgradJobs];
+};
+
+constexpr int kWgradStages = 6;
+constexpr int kWgradThreads = 512;
+
+__global__ void __launch_bounds__(kWgradThreads, 1)
+tc_wgrad_kernel(const __grid_constant__ WgradArgs args, int K, int splits, int *status) {
+    extern __shared__ unsigned char smem_raw[];
+    int j = 0;
+    while (j + 1 < kWgradJobs && (int)blockIdx.x >= args.first[j + 1]) ++j;
+    const int M = args.M[j], N = args.N[j];
+    const int at = (int)blockIdx.x - args.first[j], tiles_n = (N + 127) / 128;
+    const int m0 = at / tiles_n * kTcBM, n0 = at % tiles_n * 128;
+    const int KT_all = (K + kTcBK - 1) / kTcBK;
+    const int kt0 = (int)((long long)KT_all * blockIdx.y / splits);
+    const int kt1 = (int)((long long)KT_all * (blockIdx.y + 1) / splits);
+    const Tile<128, kWgradStages> t = setup_tile<128, kWgradStages>(smem_raw, args.a[j], args.b[j]);
+    if (tile_product(t, args.a[j], args.b[j], m0, n0, kt0, kt1 - kt0, status, 0)) {
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const int r0 = m0 + (warp & 3) * 32, col0 = n0 + (warp >> 2) * 32;
+        if (r0 < M && col0 < N) {
+            float *stg = reinterpret_cast<float *>(t.ring) + warp * (32 * kStgStride);
+            uint32_t r[32];
+            float v[32];
+            load_acc(r, t.tmem, (warp >> 2) * 32);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+            stage_f32(stg, v, lane);
+            write_f32(stg, args.out[j] + (size_t)blockIdx.y * M * N, r0, col0, M, N, N, true, false, lane);
+        }
+    }
+    release_tile<128>(t.tmem);
 }
 
 // ---- persistent variant (many output tiles, no split K) ----------------------------------
@@ -670,6 +916,76 @@ cudaError_t launch_tc_gemm(const void *A, const void *B, int M, int N, int K, co
                                             splits, s)
                    : launch_variant<128, 4>(grid, ma, mb, M, N, K, bias, act, out, out_f32, ldo, pre_out, status,
                                             splits, s);
+}
+
+namespace {
+
+template <int BN, int ST, int MODE>
+cudaError_t launch_train(const CUtensorMap &ma, const CUtensorMap &mb, int M, int N, int K, const TrainEpilogue &ep,
+                         int *status, cudaStream_t s) {
+    const int sm = TmaSmem<BN, ST>::TOTAL;
+    cudaError_t e = cudaFuncSetAttribute(tc_train_kernel<BN, ST, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    if (e != cudaSuccess) return e;
+    tc_train_kernel<BN, ST, MODE><<<dim3(M / kTcBM, (N + BN - 1) / BN), 4 * BN, sm, s>>>(ma, mb, M, N, K, ep, status);
+    return cudaGetLastError();
+}
+
+template <int BN, int ST>
+cudaError_t launch_train_mode(TrainMode mode, const CUtensorMap &ma, const CUtensorMap &mb, int M, int N, int K,
+                              const TrainEpilogue &ep, int *status, cudaStream_t s) {
+    switch (mode) {
+        case kTrainForward: return launch_train<BN, ST, kTrainForward>(ma, mb, M, N, K, ep, status, s);
+        case kTrainLoss: return launch_train<BN, ST, kTrainLoss>(ma, mb, M, N, K, ep, status, s);
+        default: return launch_train<BN, ST, kTrainBack>(ma, mb, M, N, K, ep, status, s);
+    }
+}
+
+}  // namespace
+
+cudaError_t launch_train_gemm(TrainMode mode, const void *A, const void *B, int M, int N, int K,
+                              const TrainEpilogue &ep, int *status, cudaStream_t s) {
+    if (M <= 0 || N <= 0 || K <= 0 || M % kTcBM || N % 32 || K % 8) return cudaErrorInvalidValue;
+    const int sms = sm_count_of_current_device();
+    const int nsm = sms > 0 ? sms : 152;
+    // One wave of 128-wide tiles that fill at least half of the SMs: one CTA of 16 warps per SM.
+    // Otherwise narrower tiles, two CTAs per SM: for a large batch a CTA's epilogue overlaps the
+    // other's product; for a small one, or a narrow layer, they are on more SMs.
+    const long long tm = M / kTcBM, t128 = tm * ((N + 127) / 128), t64 = tm * ((N + 63) / 64);
+    const int BN = t128 <= nsm && 2 * t128 >= nsm ? 128 : 2 * t64 >= nsm ? 64 : 32;
+    CUtensorMap ma, mb;
+    if (!make_map(&ma, A, M, K, kTcBM) || !make_map(&mb, B, N, K, BN)) return cudaErrorInvalidValue;
+    return BN == 128  ? launch_train_mode<128, 6>(mode, ma, mb, M, N, K, ep, status, s)
+           : BN == 64 ? launch_train_mode<64, 4>(mode, ma, mb, M, N, K, ep, status, s)
+                      : launch_train_mode<32, 4>(mode, ma, mb, M, N, K, ep, status, s);
+}
+
+int wgrad_splits(const WgradJob *job, int64_t K) {
+    const int sms = sm_count_of_current_device();
+    const long long nsm = sms > 0 ? sms : 152;
+    long long tiles = 0;
+    for (int j = 0; j < kWgradJobs; ++j) tiles += (long long)((job[j].M + 127) / 128) * ((job[j].N + 127) / 128);
+    // About one wave (the wave's rest is worth less than another partial sum), each part with at
+    // least four stages of K.
+    return (int)std::max(1ll, std::min<long long>(K / kTcBK / 4, nsm / std::max(1ll, tiles)));
+}
+
+cudaError_t launch_wgrad(const WgradJob *job, int K, int splits, int *status, cudaStream_t s) {
+    WgradArgs args;
+    int tiles = 0;
+    for (int j = 0; j < kWgradJobs; ++j) {
+        if (!make_map(&args.a[j], job[j].A, job[j].M, K, kTcBM) || !make_map(&args.b[j], job[j].B, job[j].N, K, 128))
+            return cudaErrorInvalidValue;
+        args.M[j] = job[j].M;
+        args.N[j] = job[j].N;
+        args.out[j] = job[j].out;
+        args.first[j] = tiles;
+        tiles += (job[j].M + 127) / 128 * ((job[j].N + 127) / 128);
+    }
+    const int sm = TmaSmem<128, kWgradStages>::TOTAL;
+    cudaError_t e = cudaFuncSetAttribute(tc_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    if (e != cudaSuccess) return e;
+    tc_wgrad_kernel<<<dim3(tiles, splits), kWgradThreads, sm, s>>>(args, K, splits, status);
+    return cudaGetLastError();
 }
 
 }  // namespace cumf
