@@ -331,61 +331,6 @@ sgd_hogwild_kernel(const UpdateArgs a) {
 // bf16-SR 2.59 -> 0.85 (to 1.12 by cvt.rs); 480,189 x 17,770, 99M, fp16 with row copies
 // 8.63 -> 8.25.
 
-// s += <p, q> over one word, in element order.  A product of two fp16 (bf16) values is exact in
-// fp32, so the mixed-precision fma rounds as the fma of the widened values does.
-template <int KIND>
-__device__ __forceinline__ float dot_word(const uint4 &p, const uint4 &q, float s) {
-    if (KIND == kFloat) {
-        using C = Conv<kFloat>;
-#pragma unroll
-        for (int h = 0; h < C::kPairs; ++h) {
-            const float2 pp = C::get(p, h), qq = C::get(q, h);
-            s = __fmaf_rn(pp.x, qq.x, s);
-            s = __fmaf_rn(pp.y, qq.y, s);
-        }
-        return s;
-    }
-#pragma unroll
-    for (int h = 0; h < 4; ++h) {
-        const uint32_t a = (&p.x)[h], b = (&q.x)[h];
-        if (KIND == kHalf)
-            asm("{.reg .f16 x, y, z, w; mov.b32 {x, y}, %1; mov.b32 {z, w}, %2;\n"
-                " fma.rn.f32.f16 %0, x, z, %0; fma.rn.f32.f16 %0, y, w, %0;}\n"
-                : "+f"(s)
-                : "r"(a), "r"(b));
-        else
-            asm("{.reg .b16 x, y, z, w; mov.b32 {x, y}, %1; mov.b32 {z, w}, %2;\n"
-                " fma.rn.f32.bf16 %0, x, z, %0; fma.rn.f32.bf16 %0, y, w, %0;}\n"
-                : "+f"(s)
-                : "r"(a), "r"(b));
-    }
-    return s;
-}
-
-__device__ __forceinline__ float2 both(float x) { return make_float2(x, x); }
-
-// update_rows for one word, two elements per instruction; nlp = -lambda_p, nlq = -lambda_q
-// (-(l*x) and (-l)*x are the same bits).
-template <int KIND, bool SR>
-__device__ __forceinline__ void update_word(const uint4 &p, const uint4 &q, uint4 &wp, uint4 &wq, float lr, float err,
-                                            float nlp, float nlq, uint32_t key, int lane) {
-    using C = Conv<KIND>;
-#pragma unroll
-    for (int h = 0; h < C::kPairs; ++h) {
-        const float2 pp = C::get(p, h), qq = C::get(q, h);
-        const float2 a = __ffma2_rn(both(lr), __ffma2_rn(both(err), qq, __fmul2_rn(both(nlp), pp)), pp);
-        const float2 b = __ffma2_rn(both(lr), __ffma2_rn(both(err), pp, __fmul2_rn(both(nlq), qq)), qq);
-        if (SR) {
-            const uint32_t pair = (uint32_t)((lane * C::kPairs + h) * 2);
-            C::put_sr(wp, h, a.x, a.y, lowbias32(key + pair));
-            C::put_sr(wq, h, b.x, b.y, lowbias32(key + pair + 1u));
-        } else {
-            C::put(wp, h, a.x, a.y);
-            C::put(wq, h, b.x, b.y);
-        }
-    }
-}
-
 // ---- popular rows -------------------------------------------------------------------------
 //
 // A row that many workers hold at once is bound by its cache lines: every store takes the line
