@@ -133,49 +133,105 @@ __global__ void import_kernel(const float *src, const int32_t *map, uint64_t row
 
 // Eight lanes per rating; float dot in fp32, squared error rounded to fp32 and summed in
 // fp64 as calc_rmse does (`mf_float e = r - z; loss += e*e;`, mf.cpp:3831-3834).
+//
+// Bound by the latency of two dependent gathers (the rating, then its rows).  So the next
+// ratings are fetched while these are summed, a group takes U ratings at a time where a row is
+// short (k = 32 C, C loads per lane and row; C = 0: any k, one at a time), and the grid is what
+// is resident at once, 5 blocks on each of 152 SMs: with 1,024 blocks a third of them ran in a
+// second wave.  1.4M ratings, 480,189 x 17,770, k = 128: 154 us, 82 so
+// (79 with 4 blocks of 64 registers, 85 with 6 of 40).
 constexpr int kRmseLanes = 8;
+constexpr int kRmsePerSm = 5;
+constexpr int kRmseBlocks = kRmsePerSm * 152;
 
-__global__ void rmse_kernel(const cumf_node *R, uint64_t nnz, const float *P, uint32_t m,
-                            const float *Q, uint32_t n, int k, float b, double *part) {
+template <int C, int U>
+__global__ void __launch_bounds__(kThreads, kRmsePerSm) rmse_kernel(const cumf_node *R, uint64_t nnz, const float *P, uint32_t m,
+                                                           const float *Q, uint32_t n, int k, float b, double *part) {
     __shared__ double sh[kThreads / 32];
     const int lane = threadIdx.x % kRmseLanes;
     const uint64_t group = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / kRmseLanes;
     const uint64_t groups = (uint64_t)gridDim.x * blockDim.x / kRmseLanes;
     const unsigned gmask = 0xffu << ((threadIdx.x & 31) & ~(kRmseLanes - 1));
     double acc = 0.0;
-    for (uint64_t i = group; i < nnz; i += groups) {
-        const cumf_node x = R[i];
-        const uint32_t u = (uint32_t)x.u, v = (uint32_t)x.v;
-        float z;
-        if (u < m && v < n) {
-            const float *p = P + (uint64_t)u * k;
-            const float *q = Q + (uint64_t)v * k;
-            float s = 0.f;
+    cumf_node next[U];
+#pragma unroll
+    for (int j = 0; j < U; ++j) {
+        next[j] = {-1, -1, 0.f};
+        if (group + j * groups < nnz) next[j] = R[group + j * groups];
+    }
+    for (uint64_t i = group; i < nnz; i += U * groups) {
+        cumf_node x[U];
+        bool ok[U];
+        float s[U];
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            x[j] = next[j];
+            next[j] = {-1, -1, 0.f};
+            const uint64_t at = i + (U + j) * groups;
+            if (at < nnz) next[j] = R[at];
+            ok[j] = (uint32_t)x[j].u < m && (uint32_t)x[j].v < n;
+            s[j] = 0.f;
+        }
+        if (C > 0) {
+            float4 p[U][C > 0 ? C : 1], q[U][C > 0 ? C : 1];
+#pragma unroll
+            for (int j = 0; j < U; ++j)
+#pragma unroll
+                for (int c = 0; c < C; ++c) {
+                    p[j][c] = q[j][c] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (ok[j]) {
+                        p[j][c] = __ldg(reinterpret_cast<const float4 *>(P + (uint64_t)(uint32_t)x[j].u * (32 * C)) + lane + kRmseLanes * c);
+                        q[j][c] = __ldg(reinterpret_cast<const float4 *>(Q + (uint64_t)(uint32_t)x[j].v * (32 * C)) + lane + kRmseLanes * c);
+                    }
+                }
+#pragma unroll
+            for (int j = 0; j < U; ++j)
+#pragma unroll
+                for (int c = 0; c < C; ++c) {
+                    s[j] = __fmaf_rn(p[j][c].x, q[j][c].x, s[j]);
+                    s[j] = __fmaf_rn(p[j][c].y, q[j][c].y, s[j]);
+                    s[j] = __fmaf_rn(p[j][c].z, q[j][c].z, s[j]);
+                    s[j] = __fmaf_rn(p[j][c].w, q[j][c].w, s[j]);
+                }
+        } else if (ok[0]) {
+            const float *p = P + (uint64_t)(uint32_t)x[0].u * k, *q = Q + (uint64_t)(uint32_t)x[0].v * k;
             if ((k & 3) == 0) {
-                const float4 *p4 = reinterpret_cast<const float4 *>(p);
-                const float4 *q4 = reinterpret_cast<const float4 *>(q);
+                const float4 *p4 = reinterpret_cast<const float4 *>(p), *q4 = reinterpret_cast<const float4 *>(q);
                 for (int c = lane; c < (k >> 2); c += kRmseLanes) {
                     const float4 a = __ldg(p4 + c), bq = __ldg(q4 + c);
-                    s = __fmaf_rn(a.x, bq.x, s);
-                    s = __fmaf_rn(a.y, bq.y, s);
-                    s = __fmaf_rn(a.z, bq.z, s);
-                    s = __fmaf_rn(a.w, bq.w, s);
+                    s[0] = __fmaf_rn(a.x, bq.x, s[0]);
+                    s[0] = __fmaf_rn(a.y, bq.y, s[0]);
+                    s[0] = __fmaf_rn(a.z, bq.z, s[0]);
+                    s[0] = __fmaf_rn(a.w, bq.w, s[0]);
                 }
             } else {
-                for (int c = lane; c < k; c += kRmseLanes) s = __fmaf_rn(__ldg(p + c), __ldg(q + c), s);
+                for (int c = lane; c < k; c += kRmseLanes) s[0] = __fmaf_rn(__ldg(p + c), __ldg(q + c), s[0]);
             }
-            for (int o = kRmseLanes / 2; o >= 1; o >>= 1) s += __shfl_xor_sync(gmask, s, o);
-            z = isnan(s) ? b : s;
-        } else {
-            z = b;
         }
-        if (lane == 0) {
-            const float e = x.r - z;
-            acc += (double)__fmul_rn(e, e);
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+#pragma unroll
+            for (int o = kRmseLanes / 2; o >= 1; o >>= 1) s[j] += __shfl_xor_sync(gmask, s[j], o);
+            if (lane == 0 && i + j * groups < nnz) {
+                const float e = x[j].r - (!ok[j] || isnan(s[j]) ? b : s[j]);
+                acc += (double)__fmul_rn(e, e);
+            }
         }
     }
     const double t = block_sum(acc, sh);
     if (threadIdx.x == 0) part[blockIdx.x] = t;
+}
+
+using RmseFn = void (*)(const cumf_node *, uint64_t, const float *, uint32_t, const float *, uint32_t, int, float,
+                        double *);
+
+RmseFn rmse_fn(int k) {
+    switch (k) {
+        case 32: return &rmse_kernel<1, 4>;
+        case 64: return &rmse_kernel<2, 2>;
+        case 128: return &rmse_kernel<4, 1>;
+        default: return &rmse_kernel<0, 1>;
+    }
 }
 
 // Sum of `count` partials in a fixed order (one block of kSumThreads): thread t adds
@@ -288,16 +344,13 @@ cudaError_t launch_export(const void *in, int precision, const int32_t *map, int
 
 int rmse_blocks(int64_t nnz) {
     (void)nnz;
-    return kReduceBlocks;
+    return kRmseBlocks;
 }
 
 cudaError_t launch_rmse(const cumf_node *d_R, int64_t nnz, const float *P, int32_t m,
                         const float *Q, int32_t n, int k, float b, double *d_part,
                         double *d_sum, cudaStream_t s) {
-    rmse_kernel<<<kReduceBlocks, kThreads, 0, s>>>(d_R, (uint64_t)nnz, P, (uint32_t)m, Q,
-                                                   (uint32_t)n, k, b, d_part);
-    sum_kernel<<<1, kSumThreads, 0, s>>>(d_part, kReduceBlocks, d_sum);
-    return cudaGetLastError();
+    return launch_rmse_grid(d_R, nnz, P, m, Q, n, k, b, kRmseBlocks, d_part, d_sum, s);
 }
 
 cudaError_t launch_import(const float *src, const int32_t *map, int64_t rows, int k, float factor, void *dst,
@@ -318,15 +371,16 @@ cudaError_t launch_import(const float *src, const int32_t *map, int64_t rows, in
 // for their code, at the first launch.
 cudaError_t load_rmse_kernels() {
     cudaFuncAttributes attr;
-    cudaError_t e = cudaFuncGetAttributes(&attr, rmse_kernel);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, sum_kernel);
+    cudaError_t e = cudaFuncGetAttributes(&attr, sum_kernel);
+    for (int k : {32, 64, 128, 0})
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, rmse_fn(k));
     return e;
 }
 
 cudaError_t launch_rmse_grid(const cumf_node *d_R, int64_t nnz, const float *P, int32_t m,
                              const float *Q, int32_t n, int k, float b, int blocks,
                              double *d_part, double *d_sum, cudaStream_t s) {
-    rmse_kernel<<<blocks, kThreads, 0, s>>>(d_R, (uint64_t)nnz, P, (uint32_t)m, Q, (uint32_t)n, k, b, d_part);
+    rmse_fn(k)<<<blocks, kThreads, 0, s>>>(d_R, (uint64_t)nnz, P, (uint32_t)m, Q, (uint32_t)n, k, b, d_part);
     sum_kernel<<<1, kSumThreads, 0, s>>>(d_part, blocks, d_sum);
     return cudaGetLastError();
 }
