@@ -322,11 +322,13 @@ struct Adam {
 };
 
 // Adam's update of element i (value w, moments m1 and m2) with gradient g; returns the new
-// value.  c1, c2: 1 - b1^t, 1 - b2^t.
+// value.  c1, c2: 1 - b1^t, 1 - b2^t.  The moments' roundings are spelled out: left to the
+// compiler's choice of fma they change with the code around them, and a last bit here travels
+// through the bf16 weights.
 __device__ __forceinline__ float adam_element(const Adam &ad, int64_t i, float g, float w, float m1, float m2,
                                               float c1, float c2) {
-    const float a = ad.b1 * m1 + (1.f - ad.b1) * g;
-    const float b = ad.b2 * m2 + (1.f - ad.b2) * g * g;
+    const float a = __fmaf_rn(1.f - ad.b1, g, __fmul_rn(ad.b1, m1));
+    const float b = __fmaf_rn(__fmul_rn(1.f - ad.b2, g), g, __fmul_rn(ad.b2, m2));
     ad.m1[i] = a;
     ad.m2[i] = b;
     w -= ad.lr * (a / c1) / (sqrtf(b / c2) + ad.eps);
@@ -342,6 +344,7 @@ struct FinishWeight {
     const float *part;  // [splits][rows][ld]
     int64_t off;
     int rows, cols, ld;  // ld >= cols: the padded columns of W1 are left out
+    int splits;
     __nv_bfloat16 *b, *bt;
 };
 struct FinishBias {
@@ -353,7 +356,7 @@ struct FinishArgs {
     FinishWeight w[3];
     FinishBias bias[3];
     int first[7];
-    int splits, tiles;  // parts of a weight gradient, of a bias gradient
+    int tiles;  // parts of a bias gradient
     float *grads;
     Adam adam;
     const double *loss_part;
@@ -433,7 +436,7 @@ __global__ void __launch_bounds__(kTile * kTileRows) finish_step_kernel(const __
     }
     if (in)
 #pragma unroll 4
-        for (int z = 1; z < args.splits; ++z)
+        for (int z = 1; z < fw.splits; ++z)
 #pragma unroll
             for (int q = 0; q < kRows; ++q) g[q] += p[z * part + (int64_t)q * kTileRows * fw.ld];
 #pragma unroll
@@ -486,17 +489,19 @@ struct Mlp {
 
 namespace {
 
-int64_t wgrad_elems(const Mlp *mp) { return (int64_t)mp->h * mp->dp + (int64_t)mp->h * mp->h + (int64_t)mp->d_out * mp->h; }
-
-// dW3 = dY^T H2, dW2 = dZ2^T H1, dW1 = dZ1^T X (padded input columns give columns that are left
-// out), with `splits` parts each in mp->wpart.
-void wgrad_jobs(Mlp *mp, int splits, WgradJob *job) {
+// dW1 = dZ1^T X (padded input columns give columns that are left out), dW2 = dZ2^T H1,
+// dW3 = dY^T H2 over rp rows, their K parts in mp->wpart.
+void wgrad_jobs(Mlp *mp, int64_t rp, WgradJob *job) {
     const int h = mp->h, dout = mp->d_out, dp = mp->dp;
-    float *w1 = mp->wpart.as<float>();
-    float *w2 = w1 + (int64_t)splits * h * dp, *w3 = w2 + (int64_t)splits * h * h;
-    job[0] = {mp->dp1t.p, mp->xbt.p, h, dp, w1};
-    job[1] = {mp->dp2t.p, mp->h1t.p, h, h, w2};
-    job[2] = {mp->dyt.p, mp->h2t.p, dout, h, w3};
+    job[0] = {mp->dp1t.p, mp->xbt.p, h, dp, 0, nullptr};
+    job[1] = {mp->dp2t.p, mp->h1t.p, h, h, 0, nullptr};
+    job[2] = {mp->dyt.p, mp->h2t.p, dout, h, 0, nullptr};
+    float *out = mp->wpart.as<float>();
+    for (int j = 0; j < kWgradJobs; ++j) {
+        job[j].splits = product_splits(job[j].M, job[j].N, rp);
+        job[j].out = out;
+        out += (int64_t)job[j].splits * job[j].M * job[j].N;
+    }
 }
 
 // Workspace for batches of up to `rows` rows: the forward buffers, and with `train` also
@@ -526,10 +531,10 @@ int mlp_ensure(Mlp *mp, int64_t rows, bool train) {
     CUMF_CUDA(mp->dp1t.alloc(r * h * b2));
     CUMF_CUDA(mp->colws.alloc((r / kTile) * (2 * h + dout) * 4));
     CUMF_CUDA(mp->lossp.alloc((r / kTile) * (dout / kTile) * sizeof(double)));
-    // The parts of the longest K that this workspace serves: fewer rows are split no further.
-    WgradJob jobs[kWgradJobs];
-    wgrad_jobs(mp, 1, jobs);
-    CUMF_CUDA(mp->wpart.alloc((size_t)wgrad_splits(jobs, r) * wgrad_elems(mp) * 4));
+    const int wm[kWgradJobs] = {h, h, dout}, wn[kWgradJobs] = {dp, h, h};
+    size_t parts = 0;
+    for (int j = 0; j < kWgradJobs; ++j) parts += (size_t)product_splits_limit(wm[j], wn[j], r) * wm[j] * wn[j];
+    CUMF_CUDA(mp->wpart.alloc(parts * 4));
     mp->cap = r;
     return CUMF_OK;
 }
@@ -636,16 +641,14 @@ int mlp_step_ws(Mlp *mp, const Batch &bt, cudaStream_t s, const Adam &adam = Ada
     CUMF_CUDA(launch_train_gemm(kTrainBack, mp->dy.p, mp->w3t.p, rp, h, dout, g2, st, s));
     CUMF_CUDA(launch_train_gemm(kTrainBack, mp->dp2.p, mp->w2t.p, rp, h, h, g1, st, s));
     WgradJob jobs[kWgradJobs];
-    wgrad_jobs(mp, 1, jobs);
-    const int splits = wgrad_splits(jobs, rp);
-    wgrad_jobs(mp, splits, jobs);
-    CUMF_CUDA(launch_wgrad(jobs, rp, splits, st, s));
+    wgrad_jobs(mp, rp, jobs);
+    CUMF_CUDA(launch_wgrad(jobs, rp, st, s));
 
     FinishArgs f{};
     auto bf = [](DevBuf &b) { return b.as<__nv_bfloat16>(); };
-    f.w[0] = {jobs[0].out, mp->off_w1, h, mp->d_in, dp, bf(mp->w1b), nullptr};
-    f.w[1] = {jobs[1].out, mp->off_w2, h, h, h, bf(mp->w2b), bf(mp->w2t)};
-    f.w[2] = {jobs[2].out, mp->off_w3, dout, h, h, bf(mp->w3b), bf(mp->w3t)};
+    f.w[0] = {jobs[0].out, mp->off_w1, h, mp->d_in, dp, jobs[0].splits, bf(mp->w1b), nullptr};
+    f.w[1] = {jobs[1].out, mp->off_w2, h, h, h, jobs[1].splits, bf(mp->w2b), bf(mp->w2t)};
+    f.w[2] = {jobs[2].out, mp->off_w3, dout, h, h, jobs[2].splits, bf(mp->w3b), bf(mp->w3t)};
     f.bias[0] = {col1, mp->off_b1, h};
     f.bias[1] = {col2, mp->off_b2, h};
     f.bias[2] = {col3, mp->off_b3, dout};
@@ -653,7 +656,6 @@ int mlp_step_ws(Mlp *mp, const Batch &bt, cudaStream_t s, const Adam &adam = Ada
         f.first[l + 1] = f.first[l] + f.w[l].rows / kTile * ((f.w[l].cols + kTile - 1) / kTile);
     }
     for (int l = 0; l < 3; ++l) f.first[l + 4] = f.first[l + 3] + f.bias[l].cols / kTile;
-    f.splits = splits;
     f.tiles = tiles;
     f.grads = mp->grads.as<float>();
     f.adam = adam;

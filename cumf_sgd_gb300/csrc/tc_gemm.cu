@@ -468,7 +468,7 @@ __device__ __forceinline__ void write_both(float *stg, const float (&v)[32], int
 // activation's arithmetic and the stores' latency, not the product (K of a few stages), are what
 // these kernels take.  Fused, because every pass over a 4096 x 512 batch between the products
 // (transposes, gelu', column sums, loss) was a launch of 2 to 8 us: a training step of 4096 rows
-// (131 -> 512 -> 512 -> 128) took 127 us of device time in 25 launches, 68 in 8.
+// (131 -> 512 -> 512 -> 128) took 127 us of device time in 25 launches, 70 in 8.
 // What the epilogue reads (slopes, targets) is fetched before the product's waits.
 template <int BN, int kStages, int MODE>
 __global__ void __launch_bounds__(4 * BN, BN == 128 ? 1 : 2)
@@ -549,30 +549,33 @@ tc_train_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     release_tile<BN>(t.tmem);
 }
 
-// The three weight gradients of a step: 128 x 128 tiles of all of them, K split so that they make
-// one wave, each part stored by itself.  One launch, since each alone leaves most SMs idle or
-// waits for its own first loads; the parts are added by the kernel that applies them, in order, so
-// that neither a zeroed output nor atomics are needed and a step gives the same bits every run.
+// The three weight gradients of a step: 128 x 128 tiles of all of them, K in the parts that each
+// product alone would have, each part stored by itself.  One launch, since each alone leaves most
+// SMs idle or waits for its own first loads; the parts are added by the kernel that applies them,
+// in order, so that neither a zeroed output nor atomics are needed and a step gives the same bits
+// every run (with one part or two, those of the product alone).
 struct WgradArgs {
     CUtensorMap a[kWgradJobs], b[kWgradJobs];
-    int M[kWgradJobs], N[kWgradJobs], first[kWgradJobs];  // first: a job's first block
+    int M[kWgradJobs], N[kWgradJobs], splits[kWgradJobs];
+    int first[kWgradJobs];  // a job's first block; its tiles follow one another, all of a part together
     float *out[kWgradJobs];
 };
 
-constexpr int kWgradStages = 6;
+constexpr int kWgradStages = 3;  // two CTAs per SM
 constexpr int kWgradThreads = 512;
 
-__global__ void __launch_bounds__(kWgradThreads, 1)
-tc_wgrad_kernel(const __grid_constant__ WgradArgs args, int K, int splits, int *status) {
+__global__ void __launch_bounds__(kWgradThreads, 2)
+tc_wgrad_kernel(const __grid_constant__ WgradArgs args, int K, int *status) {
     extern __shared__ unsigned char smem_raw[];
     int j = 0;
     while (j + 1 < kWgradJobs && (int)blockIdx.x >= args.first[j + 1]) ++j;
     const int M = args.M[j], N = args.N[j];
-    const int at = (int)blockIdx.x - args.first[j], tiles_n = (N + 127) / 128;
+    const int tiles_n = (N + 127) / 128, tiles = (M + kTcBM - 1) / kTcBM * tiles_n;
+    const int at = ((int)blockIdx.x - args.first[j]) % tiles, z = ((int)blockIdx.x - args.first[j]) / tiles;
     const int m0 = at / tiles_n * kTcBM, n0 = at % tiles_n * 128;
     const int KT_all = (K + kTcBK - 1) / kTcBK;
-    const int kt0 = (int)((long long)KT_all * blockIdx.y / splits);
-    const int kt1 = (int)((long long)KT_all * (blockIdx.y + 1) / splits);
+    const int kt0 = (int)((long long)KT_all * z / args.splits[j]);
+    const int kt1 = (int)((long long)KT_all * (z + 1) / args.splits[j]);
     const Tile<128, kWgradStages> t = setup_tile<128, kWgradStages>(smem_raw, args.a[j], args.b[j]);
     if (tile_product(t, args.a[j], args.b[j], m0, n0, kt0, kt1 - kt0, status, 0)) {
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -585,7 +588,7 @@ tc_wgrad_kernel(const __grid_constant__ WgradArgs args, int K, int splits, int *
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
             stage_f32(stg, v, lane);
-            write_f32(stg, args.out[j] + (size_t)blockIdx.y * M * N, r0, col0, M, N, N, true, false, lane);
+            write_f32(stg, args.out[j] + (size_t)z * M * N, r0, col0, M, N, N, true, false, lane);
         }
     }
     release_tile<128>(t.tmem);
@@ -862,39 +865,53 @@ int sm_count_of_current_device() {
     return sms;
 }
 
+namespace {
+
+constexpr int kShortStages = 16;
+
+struct TilePlan {
+    bool wide;
+    int splits;
+};
+
+TilePlan plan_tiles(int M, int N, int64_t K, bool plain, int nsm) {
+    const long long tiles_m = (M + kTcBM - 1) / kTcBM;
+    const int64_t kt = (K + kTcBK - 1) / kTcBK;
+    // Split K when the output has too few tiles to fill the GPU and K is long (weight
+    // gradients): about one wave of CTAs, each with at least 8 stages.
+    auto splits_for = [&](long long tiles) -> int {
+        if (!plain || kt <= kShortStages || tiles >= nsm) return 1;
+        return (int)std::max(1ll, std::min<long long>(kt / 8, nsm / tiles));
+    };
+    // 128 x 256 tiles (one A tile feeds twice the columns) unless they leave most of a wave
+    // idle: 128 x 128 tiles when those give at least 1.5 times the CTAs and the wide ones do not
+    // fill the SMs (a batch of 4096 rows has 64 wide tiles; a split is capped by K).
+    const long long tw = tiles_m * ((N + 255) / 256), tn = tiles_m * ((N + 127) / 128);
+    const long long cw = tw * splits_for(tw), cn = tn * splits_for(tn);
+    const bool wide = N > 128 && (cw >= nsm || 2 * cn < 3 * cw);
+    return {wide, splits_for(wide ? tw : tn)};
+}
+
+}  // namespace
+
 cudaError_t launch_tc_gemm(const void *A, const void *B, int M, int N, int K, const float *bias, int act,
                            void *out, int out_f32, int ldo, float *pre_out, int *status, cudaStream_t s) {
     if (M <= 0 || N <= 0 || K <= 0 || (K % 8) != 0) return cudaErrorInvalidValue;
     if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return cudaErrorInvalidValue;
     const int sms = sm_count_of_current_device();
-    const int nsm = sms > 0 ? sms : 152;
     const int tiles_m = (M + kTcBM - 1) / kTcBM;
     const int kt = (K + kTcBK - 1) / kTcBK;
     // Short K (at most 16 stages of 64): a 2-stage ring, so two CTAs share an SM and
     // one CTA's epilogue overlaps another's loads.  Long K: a 4-stage ring, one CTA per SM.
-    const bool short_k = kt <= 16;
-    // Split K when the output has too few tiles to fill the GPU and K is long (weight
-    // gradients): about one wave of CTAs, each with at least 8 stages.
+    const bool short_k = kt <= kShortStages;
     const bool plain = out_f32 && !bias && act == 0 && !pre_out;
-    auto splits_for = [&](long long tiles) -> int {
-        if (!plain || short_k || tiles >= nsm) return 1;
-        return (int)std::max(1ll, std::min<long long>(kt / 8, nsm / tiles));
-    };
-    // 128 x 256 tiles (one A tile feeds twice the columns) unless they leave most of a wave
-    // idle: 128 x 128 tiles when those give at least 1.5 times the CTAs and the wide ones do not
-    // fill the SMs (the MLP's 4096-row batches: 64 wide tiles, or weight gradients whose split
-    // is capped by K).
-    bool wide = N > 128;
-    if (wide) {
-        const long long tw = (long long)tiles_m * ((N + 255) / 256), tn = (long long)tiles_m * ((N + 127) / 128);
-        const long long cw = tw * splits_for(tw), cn = tn * splits_for(tn);
-        wide = cw >= nsm || 2 * cn < 3 * cw;
-    }
+    const TilePlan plan = plan_tiles(M, N, K, plain, sms > 0 ? sms : 152);
+    const bool wide = plan.wide;
     const int BN = wide ? 256 : 128;
     CUtensorMap ma, mb;
     if (!make_map(&ma, A, M, K, kTcBM) || !make_map(&mb, B, N, K, BN)) return cudaErrorInvalidValue;
     const int tiles_n = (N + BN - 1) / BN;
-    const int splits = splits_for((long long)tiles_m * tiles_n);
+    const int splits = plan.splits;
     if (splits > 1) {
         cudaError_t e = cudaMemset2DAsync(out, (size_t)ldo * 4, 0, (size_t)N * 4, M, s);
         if (e != cudaSuccess) return e;
@@ -959,32 +976,34 @@ cudaError_t launch_train_gemm(TrainMode mode, const void *A, const void *B, int 
                       : launch_train_mode<32, 4>(mode, ma, mb, M, N, K, ep, status, s);
 }
 
-int wgrad_splits(const WgradJob *job, int64_t K) {
+int product_splits(int M, int N, int64_t K) {
     const int sms = sm_count_of_current_device();
-    const long long nsm = sms > 0 ? sms : 152;
-    long long tiles = 0;
-    for (int j = 0; j < kWgradJobs; ++j) tiles += (long long)((job[j].M + 127) / 128) * ((job[j].N + 127) / 128);
-    // About one wave (the wave's rest is worth less than another partial sum), each part with at
-    // least four stages of K.
-    return (int)std::max(1ll, std::min<long long>(K / kTcBK / 4, nsm / std::max(1ll, tiles)));
+    return plan_tiles(M, N, K, true, sms > 0 ? sms : 152).splits;
 }
 
-cudaError_t launch_wgrad(const WgradJob *job, int K, int splits, int *status, cudaStream_t s) {
+int product_splits_limit(int M, int N, int64_t K) {
+    const int sms = sm_count_of_current_device();
+    const long long fewest = (long long)((M + kTcBM - 1) / kTcBM) * ((N + 255) / 256);
+    return (int)std::max<long long>(1, std::min<long long>(K / kTcBK / 8, (sms > 0 ? sms : 152) / fewest));
+}
+
+cudaError_t launch_wgrad(const WgradJob *job, int K, int *status, cudaStream_t s) {
     WgradArgs args;
-    int tiles = 0;
+    int blocks = 0;
     for (int j = 0; j < kWgradJobs; ++j) {
         if (!make_map(&args.a[j], job[j].A, job[j].M, K, kTcBM) || !make_map(&args.b[j], job[j].B, job[j].N, K, 128))
             return cudaErrorInvalidValue;
         args.M[j] = job[j].M;
         args.N[j] = job[j].N;
+        args.splits[j] = job[j].splits;
         args.out[j] = job[j].out;
-        args.first[j] = tiles;
-        tiles += (job[j].M + 127) / 128 * ((job[j].N + 127) / 128);
+        args.first[j] = blocks;
+        blocks += (job[j].M + 127) / 128 * ((job[j].N + 127) / 128) * job[j].splits;
     }
     const int sm = TmaSmem<128, kWgradStages>::TOTAL;
     cudaError_t e = cudaFuncSetAttribute(tc_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
     if (e != cudaSuccess) return e;
-    tc_wgrad_kernel<<<dim3(tiles, splits), kWgradThreads, sm, s>>>(args, K, splits, status);
+    tc_wgrad_kernel<<<blocks, kWgradThreads, sm, s>>>(args, K, status);
     return cudaGetLastError();
 }
 

@@ -32,15 +32,18 @@ struct TrainEpilogue {
 cudaError_t launch_train_gemm(TrainMode mode, const void *A, const void *B, int M, int N, int K,
                               const TrainEpilogue &ep, int *status, cudaStream_t s);
 
-// Up to three products C_j[M_j x N_j] = A_j[M_j x K] B_j[N_j x K]^T over the same long K in one
-// launch, K in `splits` parts: out_j[splits][M_j][N_j] (fp32) are the parts' sums.
+// Three products C_j[M_j x N_j] = A_j[M_j x K] B_j[N_j x K]^T over the same K in one launch, K in
+// `splits` parts each: out[splits][M][N] (fp32) are the parts' sums.
 struct WgradJob {
     const void *A, *B;
-    int M, N;
+    int M, N, splits;
     float *out;
 };
 constexpr int kWgradJobs = 3;
-int wgrad_splits(const WgradJob *job, int64_t K);
-cudaError_t launch_wgrad(const WgradJob *job, int K, int splits, int *status, cudaStream_t s);
+// The parts that launch_tc_gemm would add for a plain fp32 product, and the most that it would for
+// any K up to this one.
+int product_splits(int M, int N, int64_t K);
+int product_splits_limit(int M, int N, int64_t K);
+cudaError_t launch_wgrad(const WgradJob *job, int K, int *status, cudaStream_t s);
 
 }  // namespace cumf
