@@ -109,9 +109,9 @@ def hot_rows_of(args) -> float:
 # row copies, no L2 prefetch), from one ncu capture of this kernel.  A constant: ncu cannot run
 # inside the timed bench, and the capture is redone whenever the kernel or the defaults change;
 # other configurations report no traffic.
-UPDATE_KERNEL_DRAM_BYTES_C2 = 18.341e9
-UPDATE_KERNEL_DRAM_BYTES_SOURCE = ("ncu capture of one c2 fp16 launch of sgd_hogwild_kernel<128,fp16,16>, "
-                                   "97,280 workers, row copies, prefetch 0: 9.057 GB read + 9.284 GB written")
+UPDATE_KERNEL_DRAM_BYTES_C2 = 18.074e9
+UPDATE_KERNEL_DRAM_BYTES_SOURCE = ("ncu capture of one c2 fp16 launch of sgd_pair_kernel<128,fp16,16>, "
+                                   "97,280 workers, row copies, prefetch 0: 8.870 GB read + 9.204 GB written")
 
 
 class ClockSampler:
