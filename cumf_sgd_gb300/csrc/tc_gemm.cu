@@ -600,33 +600,34 @@ tc_wgrad_kernel(const __grid_constant__ WgradArgs args, int K, int *status) {
 // m-block are adjacent, so their A rows are read once from DRAM).  Warp 0 (one lane) streams
 // operand stages through the ring across tile boundaries; warp 1 (one lane) issues the MMAs
 // into one of two tensor-memory accumulators (tile j uses accumulator j % 2) and commits
-// `tfull`; warps 2-17 drain an accumulator (tcgen05.ld, bias, activation, staged coalesced
-// stores), four to a tensor-memory lane quarter, and release it through `tempty` while the next
-// tile's MMAs fill the other one.  The epilogue is what bounds it (an activation is some fifty
-// instructions per output): at 50,000 x 512 outputs with gelu four epilogue warps took 85 us per
-// product, eight 53, sixteen 46.  Their staging blocks take one stage of the 256-wide ring and
-// two of the 128-wide one, which K of a few stages does not miss.
-constexpr int kPersEpilogueWarps = 16;
-constexpr int kPersThreads = 64 + 32 * kPersEpilogueWarps;
-
-template <int BN, int kStages>
+// `tfull`; kWarps more drain an accumulator (tcgen05.ld, bias, activation, staged coalesced
+// stores), kWarps / 4 to a tensor-memory lane quarter, and release it through `tempty` while the
+// next tile's MMAs fill the other one.
+//
+// Up to some 26 stages of K the epilogue is what bounds it (an activation is some fifty
+// instructions per output): sixteen warps; at 50,000 x 512 outputs with gelu, K = 512, four
+// epilogue warps took 85 us per product, eight 53, sixteen 46.  Their staging blocks take one
+// stage of the 256-wide ring and two of the 128-wide one, which a longer product misses: four
+// warps and the longer ring from there on.  65,536 x 512 outputs, bf16, sixteen / four: K = 1536
+// 88 / 95 us, K = 2048 112 / 101; 16,384 x 4096: K = 2048 191 / 203, K = 3072 277 / 235.
+template <int BN, int kStages, int kWarps>
 struct PersSmem {
     static constexpr int A_BYTES = kTcBM * 128;
     static constexpr int B_BYTES = BN * 128;
     static constexpr int STAGE = A_BYTES + B_BYTES;
-    static constexpr int STG = kPersEpilogueWarps * 32 * kStgStride * 4;  // the epilogue warps' staging blocks
+    static constexpr int STG = kWarps * 32 * kStgStride * 4;  // the epilogue warps' staging blocks
     static constexpr int TOTAL = 1024 + kStages * STAGE + STG + 256;
     static_assert(TOTAL <= 232448, "shared memory of one CTA");
 };
 
 __device__ __forceinline__ bool aborted(const int *flag) { return *reinterpret_cast<const volatile int *>(flag) != 0; }
 
-template <int BN, int kStages>
-__global__ void __launch_bounds__(kPersThreads, 1)
+template <int BN, int kStages, int kWarps>
+__global__ void __launch_bounds__(64 + 32 * kWarps, 1)
 tc_gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, int M,
                           int N, int K, const float *__restrict__ bias, int act, void *out, int out_f32, int ldo,
                           float *pre_out, int *status) {
-    using S = PersSmem<BN, kStages>;
+    using S = PersSmem<BN, kStages, kWarps>;
     extern __shared__ unsigned char smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;  // swizzle atoms need 1024-byte alignment
@@ -654,7 +655,7 @@ tc_gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
         for (int i = 0; i < 2; ++i) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&tfull[i])));
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&tempty[i])),
-                         "n"(kPersEpilogueWarps));  // one arrival per epilogue warp
+                         "n"(kWarps));  // one arrival per epilogue warp
         }
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(mma_done)));
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -739,9 +740,9 @@ tc_gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
                              smem_u32(mma_done))
                          : "memory");
         }
-    } else {  // epilogue warps: tensor-memory lanes 32 (warp % 4).., a quarter of the columns each
+    } else {  // epilogue warps: tensor-memory lanes 32 (warp % 4).., kCols columns each
         const int quarter = warp & 3, part = (warp - 2) >> 2;
-        constexpr int kCols = BN / (kPersEpilogueWarps / 4);
+        constexpr int kCols = BN / (kWarps / 4);
         float *stg = stg_all + (warp - 2) * (32 * kStgStride);
         for (int j = 0; j < my_tiles; ++j) {
             const int acc = j & 1;
@@ -843,15 +844,15 @@ cudaError_t launch_variant(dim3 grid, const CUtensorMap &ma, const CUtensorMap &
     return cudaGetLastError();
 }
 
-template <int BN, int ST>
+template <int BN, int ST, int EW>
 cudaError_t launch_persistent(int grid, const CUtensorMap &ma, const CUtensorMap &mb, int M, int N, int K,
                               const float *bias, int act, void *out, int out_f32, int ldo, float *pre_out, int *status,
                               cudaStream_t s) {
-    const int sm = PersSmem<BN, ST>::TOTAL;
+    const int sm = PersSmem<BN, ST, EW>::TOTAL;
     cudaError_t e =
-        cudaFuncSetAttribute(tc_gemm_persistent_kernel<BN, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+        cudaFuncSetAttribute(tc_gemm_persistent_kernel<BN, ST, EW>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
     if (e != cudaSuccess) return e;
-    tc_gemm_persistent_kernel<BN, ST><<<grid, kPersThreads, sm, s>>>(ma, mb, M, N, K, bias, act, out, out_f32, ldo,
+    tc_gemm_persistent_kernel<BN, ST, EW><<<grid, 64 + 32 * EW, sm, s>>>(ma, mb, M, N, K, bias, act, out, out_f32, ldo,
                                                                      pre_out, status);
     return cudaGetLastError();
 }
@@ -868,6 +869,7 @@ int sm_count_of_current_device() {
 namespace {
 
 constexpr int kShortStages = 16;
+constexpr int kEpilogueBoundStages = 26;
 
 struct TilePlan {
     bool wide;
@@ -920,8 +922,12 @@ cudaError_t launch_tc_gemm(const void *A, const void *B, int M, int N, int K, co
     // next tiles' loads and MMAs.
     if (splits == 1 && sms > 0 && (long long)tiles_m * tiles_n >= 2ll * sms) {
         const int g = std::min(tiles_m * tiles_n, sms);
-        return wide ? launch_persistent<256, 3>(g, ma, mb, M, N, K, bias, act, out, out_f32, ldo, pre_out, status, s)
-                    : launch_persistent<128, 4>(g, ma, mb, M, N, K, bias, act, out, out_f32, ldo, pre_out, status, s);
+        // (see the kernel: what a tile's epilogue takes, its product has to cover)
+        if (kt <= kEpilogueBoundStages)
+            return wide ? launch_persistent<256, 3, 16>(g, ma, mb, M, N, K, bias, act, out, out_f32, ldo, pre_out, status, s)
+                        : launch_persistent<128, 4, 16>(g, ma, mb, M, N, K, bias, act, out, out_f32, ldo, pre_out, status, s);
+        return wide ? launch_persistent<256, 4, 4>(g, ma, mb, M, N, K, bias, act, out, out_f32, ldo, pre_out, status, s)
+                    : launch_persistent<128, 6, 4>(g, ma, mb, M, N, K, bias, act, out, out_f32, ldo, pre_out, status, s);
     }
     const dim3 grid(tiles_m, tiles_n, splits);
     if (wide)
@@ -968,7 +974,7 @@ cudaError_t launch_train_gemm(TrainMode mode, const void *A, const void *B, int 
     // Otherwise narrower tiles, two CTAs per SM: for a large batch a CTA's epilogue overlaps the
     // other's product; for a small one, or a narrow layer, they are on more SMs.
     const long long tm = M / kTcBM, t128 = tm * ((N + 127) / 128), t64 = tm * ((N + 63) / 64);
-    const int BN = t128 <= nsm && 2 * t128 >= nsm ? 128 : 2 * t64 >= nsm ? 64 : 32;
+    const int BN = N > 64 && t128 <= nsm && 2 * t128 >= nsm ? 128 : 2 * t64 >= nsm ? 64 : 32;
     CUtensorMap ma, mb;
     if (!make_map(&ma, A, M, K, kTcBM) || !make_map(&mb, B, N, K, BN)) return cudaErrorInvalidValue;
     return BN == 128  ? launch_train_mode<128, 6>(mode, ma, mb, M, N, K, ep, status, s)
