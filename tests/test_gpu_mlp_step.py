@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("rows,d_in,h,d_out", [(1, 5, 64, 64), (127, 64, 64, 64), (129, 131, 192, 64),
                                                (640, 35, 512, 128), (2500, 131, 512, 192), (5000, 67, 512, 128),
-                                               (4097, 131, 128, 256), (12000, 16, 64, 64)])
+                                               (4097, 131, 128, 256), (12000, 16, 64, 64), (11000, 20, 1024, 64)])
 def test_mlp_step_gradients_match_fp64(lib, cuda, rows, d_in, h, d_out):
     import torch
     rng = np.random.default_rng(rows + h)
