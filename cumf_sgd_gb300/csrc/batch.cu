@@ -111,7 +111,6 @@ __device__ __forceinline__ void store_slice(char *p, const Slice<SB> &s) {
 }
 
 __device__ __forceinline__ float2 widen(uint32_t w) { return __half22float2(*reinterpret_cast<__half2 *>(&w)); }
-__device__ __forceinline__ float2 both(float x) { return make_float2(x, x); }
 
 // <p, q> over one slice, in element order.  A product of two fp16 values is exact in fp32, so the
 // mixed-precision fma rounds as the fma of the widened values does.
