@@ -230,7 +230,9 @@ __device__ __forceinline__ int64_t count_greater(const float *s, int64_t len, fl
 // feed 16 x kSweepCols FMAs), two rows per fma.rn.f32x2.  The rows' sorted predictions are
 // searched in shared memory where they fit (pred_cap floats for the 16 rows), without branches:
 // a row's length is the same for all threads.  10,000 x 2,000, k = 128, 70,000 positives:
-// 445 -> 215 us (one column per thread, one 4-byte broadcast per FMA, searches in L1 before).
+// 445 -> 260 us (one column per thread, one 4-byte broadcast per FMA, searches in L1 before).
+// Four columns per thread (162 registers) take 497 us, a group's columns over several blocks 388:
+// a block's set-up, four dependent loads, is a quarter of its time.
 constexpr int kSweepCols = 2;
 constexpr int kSweepPreds = 1024;
 
