@@ -284,7 +284,7 @@ int cumf_hot_rows_plan(const cumf_node *d_R, int64_t nnz, int32_t m, int32_t n, 
     h->grp_m = reinterpret_cast<int32_t *>(base + b_tm + b_tn);
     h->grp_n = reinterpret_cast<int32_t *>(base + b_tm + b_tn + b_gm);
     DevBuf cnt;
-    e = cnt.alloc(((size_t)m + n) * sizeof(unsigned long long) + 4 * sizeof(long long), s);
+    e = cnt.alloc(((size_t)m + n) * sizeof(unsigned long long) + 4 * sizeof(long long));
     if (e != cudaSuccess) return bail(cuda_fail(e, "hot_rows_plan: counts"));
     unsigned long long *cnt_m = cnt.as<unsigned long long>(), *cnt_n = cnt_m + m;
     long long *d_tot = reinterpret_cast<long long *>(cnt_n + n);

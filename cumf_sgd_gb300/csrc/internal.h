@@ -74,11 +74,12 @@ bool lanes_supported(int k, int precision, int lanes);
 // automatic worker count (1024 threads per SM; 0 without a device or kernel).
 int resident_workers(int k, int precision, int lanes, int sm_count);
 int wave_workers(int k, int precision, int lanes, int sm_count);
+// d_flags: 8 bytes of scratch in the stream's order (NULL: taken from the library's pool).
 cudaError_t launch_sgd_update(const cumf_node *d_R, int64_t nnz, void *d_P, int32_t m,
                               void *d_Q, int32_t n, int k, int precision, int num_workers,
                               const Tuning &tuning, const float *d_lr, int first_epoch,
                               int n_epochs, float lambda_p, float lambda_q, uint64_t seed,
-                              int *d_status, cudaStream_t stream, int *lanes_used);
+                              int *d_status, cudaStream_t stream, int *lanes_used, void *d_flags = nullptr);
 
 // ---- prep.cu ---------------------------------------------------------------------------
 // index_offset: element index of d[0] in the whole matrix (segments of modes B/C draw the

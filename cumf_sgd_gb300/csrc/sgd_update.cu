@@ -14,10 +14,9 @@
 // 16-byte ld.global.cg / st.global.cg, so a k=128 fp16 row (256 B) is one vector per lane
 // of a 16-lane group and two workers share a warp.  The dot product is a butterfly of
 // shfl.xor within the group (every lane ends with the same bits).  Two kernels:
-//   sgd_pair_kernel     one 16-byte word per lane (every default width but fp32 k = 256): two
-//                       records at a time;
-//   sgd_hogwild_kernel  two or more words per lane: one record at a time, the next one's rows in
-//                       flight.
+//   sgd_hogwild_kernel  one record at a time, the next one's rows in flight;
+//   sgd_pair_kernel     two records at a time, where a lane holds one 16-byte word of a row (every
+//                       default width but fp32 k = 256) and no row is much contended.
 // Either way a worker applies its records strictly in order: a row that an earlier record has
 // just written is forwarded to a record whose loads were issued before the store.  Records
 // are staged 32 (narrow groups: 16) at a time through shared memory (4-byte cp.async copies of
@@ -36,11 +35,10 @@ namespace {
 
 constexpr int kBlock = 256;   // threads per block
 constexpr int kMinBlocks = 4; // >= 1024 resident threads per SM (<= 64 registers)
-// Threads per block and blocks per SM of sgd_pair_kernel: 1024 threads per SM (64 registers), 896
-// (72 registers) when popular rows are told apart, or 640 (96 registers) in smaller blocks with
-// stochastic rounding.
+// Threads per block and blocks per SM of sgd_pair_kernel: 1024 threads per SM (64 registers), or
+// 640 (96 registers) in smaller blocks with stochastic rounding.
 constexpr int pair_block(bool sr) { return sr ? 64 : 128; }
-constexpr int pair_min_blocks(bool sr, bool hot) { return sr ? 10 : hot ? 7 : 8; }
+constexpr int pair_min_blocks(bool sr) { return sr ? 10 : 8; }
 // Threads per SM that a wave of workers stands for (cumf_default_workers): part of the sample
 // schedule through the automatic worker count, so it stays whatever a kernel's occupancy is.
 constexpr int kWaveThreads = 1024;
@@ -68,8 +66,16 @@ struct UpdateArgs {
     int prefetch;   // rows of record j+prefetch are pulled into L2 while record j runs (0 = off)
     int hints;      // 1 = L2 eviction hints (ratings evict_first, factor rows evict_last)
     int freeze_q;   // 1 = item rows are read but never written (user-side fold-in)
-    const uint32_t *hot;  // bit sets of the popular users and items (sample_popular_kernel), or NULL
+    const uint2 *contended;  // users' and items' flags of sample_rows_kernel, or NULL: run
+    int run_contended;       // run if either flag is set (1) or if neither is (0)
 };
+
+// Of the two launches that follow sample_rows_kernel, the other one runs.
+__device__ __forceinline__ bool skip_launch(const UpdateArgs &a) {
+    if (a.contended == nullptr) return false;
+    const uint2 f = __ldg(a.contended);
+    return ((f.x | f.y) != 0) != (a.run_contended != 0);
+}
 
 // Copy of a word the compiler cannot see through: the update phase re-widens the packed
 // rows instead of keeping the dot phase's fp32 copies alive across the group reduction.
@@ -128,6 +134,7 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 template <int K, int KIND, int G, bool SR>
 __global__ void __launch_bounds__(kBlock, kMinBlocks)
 sgd_hogwild_kernel(const UpdateArgs a) {
+    if (skip_launch(a)) return;
     using C = Conv<KIND>;
     constexpr int SB = store_bytes(KIND);
     constexpr int ROW_WORDS = K * SB / 16;          // uint4 words per row
@@ -320,53 +327,58 @@ sgd_hogwild_kernel(const UpdateArgs a) {
 // (four records) is faster still (3,000 x 1,200: 0.25 ms) but loses twice the updates on popular
 // rows: 10,000 x 2,000, 0.9M ratings, Zipf 1.0, 20 epochs, test RMSE 0.8069 at 878 workers and
 // 0.905 at 7,904, against 0.8038 and 0.842 as here (0.8030 and 0.841 one record at a time).
-// With the GPU full the epoch is bound by L2 (and, without row copies, by the queues on popular
-// rows): what pays there is fewer instructions per record (no zero fill, no register moves, no
-// forwarding; fp16 and bf16 products accumulate by mixed-precision fma, exact as the widened
-// ones; f32x2 pairs in the update).  1024 threads per SM: with 80 registers and 768 threads an
-// epoch with row copies takes 8.36 ms, 8.25 here.  The random bits of stochastic rounding want
-// 96 registers (0.93 ms with 64, and 0.98 in blocks of 128).
+// With the GPU full the epoch is bound by L2: what pays there is fewer instructions per record (no
+// zero fill, no register moves, no forwarding; fp16 and bf16 products accumulate by
+// mixed-precision fma, exact as the widened ones; f32x2 pairs in the update).  1024 threads per
+// SM: with 80 registers and 768 threads an epoch with row copies takes 8.36 ms, 8.25 here.  The
+// random bits of stochastic rounding want 96 registers (0.93 ms with 64, and 0.98 in blocks of 128).
 // Measured per epoch on GB300 against one record at a time: 300 x 120, 20,000 ratings, fp32
 // 0.41 -> 0.23 ms; 3,000 x 1,200, 200,000, fp16 0.56 -> 0.35; 120,047 x 62,501, 12.4M, k = 64,
 // bf16-SR 2.59 -> 0.85 (to 1.12 by cvt.rs); 480,189 x 17,770, 99M, fp16 with row copies
 // 8.63 -> 8.25.
 
-// ---- popular rows -------------------------------------------------------------------------
+// ---- contended rows -----------------------------------------------------------------------
 //
-// A row that many workers hold at once is bound by its cache lines: every store takes the line
-// from the SMs that read it, and the next load fetches it back, about 150 ns a turn.  A 16-byte
-// atomic exchange writes at the line's home in L2 instead and spares the turns.  Measured,
-// random read-modify-writes of H rows of 256 bytes by 9,728 workers, ns per row, store /
-// exchange: H = 8 3.6 / 2.6, 64 1.05 / 0.46, 512 0.31 / 0.17, 17,770 0.060 / 0.080.  So rows
-// that about kPopularWorkers records in flight name at a time are written by exchange (the same
-// bits either way), the others by plain stores.  Per epoch, with all stores plain / this rule:
-// 480,189 x 17,770, 99M ratings, fp16 14.2 / 10.4 ms (60 items, 4% of the ratings; at 4 workers
-// 10.3, at 2 10.6, every row 16.5); 10,000 x 2,000, 0.9M, Zipf 1.0 2.55 / 0.83; 240,000 x
-// 17,770, 50M, fp32 10.0 / 9.2.
-// Which rows those are is sampled before the launch: up to 2 ratings per record in flight are
-// counted by hashed id, and the ids whose count reaches the limit form two bit sets that the
-// update kernel keeps in shared memory.  The bits only choose the store instruction: a wrong one
-// costs time, never a result.  With few records in flight the exchanges' own latency costs more
-// than the turns: fp16, Zipf 1.0 as above, 256 workers 1.85 ms plain, 1.9-2.1 by exchange, 512
-// workers 2.36, 1.12; 3,000 x 1,200 at 390 records in flight 0.36 plain, 0.42 with the rule; and
-// the longer chains of stochastic rounding queue later (30,000 x 6,000, k = 64, bf16-SR, 878
-// workers 1.8 plain, 2.25 by exchange; 2,048 workers 1.83, 1.12).
-constexpr int kPopularBits = 14;  // hashed ids per side: 16,384 (unpopular ids share few hits)
-constexpr int kPopularWords = (1 << kPopularBits) / 32;
-constexpr int kPopularWorkers = 8;
+// A row that many workers hold at once is bound by its cache lines, and of the updates that meet
+// on it some are lost: which ones depends on how long a record is between load and store, so the
+// two kernels leave such rows at other values.  How far two records at a time are from one, as a
+// multiple of how far two runs of one are apart (medians over 36 pairs of runs of the largest
+// entry difference of P or Q; 10,000 x 2,000, 0.9M ratings, 878 workers, 15 epochs from a trained
+// model, T records in flight on the most popular row):
+//      T     fp16, k = 32 / 64 / 128 / 256     fp32, k = 32 / 64 / 128
+//      2     1.1  1.1  1.1  1.2                1.3  1.3  1.2
+//      5     1.1  1.2  1.2  1.4                1.2  1.4  1.5
+//      17    1.1  1.1  1.4  1.4                1.2  2.4  1.7
+//      28    1.1  1.0  2.1  1.7                1.2  1.4  2.4
+//      73    1.0  1.1  2.5  3.1                1.3  3.2  2.1
+// (stochastic rounding, k = 128 and 256: at most 1.3 up to 28, 2.3 at 73).  Nor are two records at a
+// time faster on wide rows there: fp16, k = 128, 7.2 ms for 9.6 at T = 17, 9.9 for 9.8 at 28, 19.9
+// for 20.7 at 73.  So a launch takes one record at a time when a row is named by more than
+// contended_limit records in flight.  Whether one is, is sampled on the device before the launch
+// (some thousand ratings counted by hashed id, about 10 us), and of the two launches that follow
+// one returns at once.
+// A 16-byte atomic exchange instead of the store spares a popular row the turns of its lines
+// (480,189 x 17,770, 99M ratings, fp16, 14.2 -> 10.4 ms), but loses other updates again: 10 epochs
+// there leave Q 1.8 times as far off, 20 epochs at T = 160 P 3.3 times.
+constexpr int kIdBits = 14;  // hashed ids per side: 16,384 (unpopular ids share few hits)
 constexpr int kSampleThreads = 1024;
-constexpr int kMaxSamples = 16384;
+constexpr int kLimitHits = 16;      // samples that a limit stands for
+constexpr int kMinHits = 12;        // with fewer, chance would decide
+constexpr int kMaxSamples = 32768;  // < 2^16: 16-bit counters, two to a word
 
-__device__ __forceinline__ uint32_t popular_hash(uint32_t id) { return (id * 0x9E3779B1u) >> (32 - kPopularBits); }
+// Rows of one cache line stand more (up to 73 as above, and there two records at a time are still
+// faster: fp16, k = 64, 10.7 ms for 12.7), and so do rows that random rounding moves as far anyway.
+constexpr int contended_limit(int row_bytes, bool sr) { return row_bytes <= 128 ? 64 : sr ? 16 : 4; }
 
-constexpr int popular_min_in_flight(bool sr) { return sr ? 4096 : 1024; }
+__device__ __forceinline__ uint32_t id_hash(uint32_t id) { return (id * 0x9E3779B1u) >> (32 - kIdBits); }
 
-// Block 0: users, block 1: items.  `samples` < 2^16 (16-bit counters, two to a word).
-__global__ void __launch_bounds__(kSampleThreads) sample_popular_kernel(const cumf_node *R, uint64_t nnz, uint32_t m,
-                                                                        uint32_t n, int samples, uint32_t limit,
-                                                                        uint64_t key, uint32_t *bits) {
-    __shared__ uint32_t cnt[(1 << kPopularBits) / 2];
-    for (int i = threadIdx.x; i < (1 << kPopularBits) / 2; i += kSampleThreads) cnt[i] = 0;
+// Block 0: users, block 1: items (n = 0: item rows are not written).  flags[block] = an id was
+// drawn `limit` times or more.
+__global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(const cumf_node *R, uint64_t nnz, uint32_t m,
+                                                                     uint32_t n, int samples, uint32_t limit,
+                                                                     uint64_t key, uint32_t *flags) {
+    __shared__ uint32_t cnt[(1 << kIdBits) / 2];
+    for (int i = threadIdx.x; i < (1 << kIdBits) / 2; i += kSampleThreads) cnt[i] = 0;
     __syncthreads();
     const uint32_t rows = blockIdx.x == 0 ? m : n;
     const uint32_t *const ids = reinterpret_cast<const uint32_t *>(R) + blockIdx.x;
@@ -374,36 +386,21 @@ __global__ void __launch_bounds__(kSampleThreads) sample_popular_kernel(const cu
     for (int i = threadIdx.x; i < samples; i += kSampleThreads) {
         const uint32_t id = __ldg(ids + 3 * mulhi64(splitmix64(key + (uint64_t)i), nnz));
         if (id < rows) {
-            const uint32_t h = popular_hash(id);
+            const uint32_t h = id_hash(id);
             atomicAdd(&cnt[h >> 1], 1u << ((h & 1) * 16));
         }
     }
     __syncthreads();
-    if (threadIdx.x < kPopularWords) {
-        uint32_t w = 0;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const uint32_t c = cnt[threadIdx.x * 16 + i];
-            w |= (uint32_t)((c & 0xffffu) >= limit) << (2 * i) | (uint32_t)((c >> 16) >= limit) << (2 * i + 1);
-        }
-        bits[blockIdx.x * kPopularWords + threadIdx.x] = w;
-    }
+    int over = 0;
+    for (int i = threadIdx.x; i < (1 << kIdBits) / 2; i += kSampleThreads)
+        over |= (cnt[i] & 0xffffu) >= limit || (cnt[i] >> 16) >= limit;
+    over = __syncthreads_or(over);
+    if (threadIdx.x == 0) flags[blockIdx.x] = over != 0;
 }
 
-__device__ __forceinline__ void store_row(uint4 *p, uint4 v, uint64_t pol, uint32_t popular) {
-    if (popular) {
-        const uint64_t lo = (uint64_t)v.x | ((uint64_t)v.y << 32), hi = (uint64_t)v.z | ((uint64_t)v.w << 32);
-        asm volatile("{.reg .b128 x, y; mov.b128 x, {%1, %2}; atom.relaxed.gpu.global.exch.b128 y, [%0], x;}\n" ::"l"(p),
-                     "l"(lo), "l"(hi)
-                     : "memory");
-    } else {
-        st_row_hint(p, v, pol);
-    }
-}
-
-// HOT: the launch has popular rows to tell apart (a.hot); item rows are not frozen.
-template <int K, int KIND, int G, bool SR, bool HOT>
-__global__ void __launch_bounds__(pair_block(SR), pair_min_blocks(SR, HOT)) sgd_pair_kernel(const UpdateArgs a) {
+template <int K, int KIND, int G, bool SR>
+__global__ void __launch_bounds__(pair_block(SR), pair_min_blocks(SR)) sgd_pair_kernel(const UpdateArgs a) {
+    if (skip_launch(a)) return;
     constexpr int ROW_WORDS = K * store_bytes(KIND) / 16;
     static_assert(ROW_WORDS == G, "one word per lane");
     constexpr int kChunk = chunk_of(G);
@@ -414,17 +411,6 @@ __global__ void __launch_bounds__(pair_block(SR), pair_min_blocks(SR, HOT)) sgd_
     // Two chunks per group, records as they are in memory; the odd stride keeps the groups of a
     // warp on different banks.
     __shared__ uint32_t s_rec[pair_block(SR) / G][2 * CW + 1];
-    __shared__ uint32_t s_popular[2][HOT ? kPopularWords : 1];  // users, items
-    int any_popular = 0;
-    if (HOT) {
-        for (int i = threadIdx.x; i < 2 * kPopularWords; i += pair_block(SR)) {
-            const uint32_t w = __ldg(a.hot + i);
-            (&s_popular[0][0])[i] = w;
-            any_popular |= w != 0;
-        }
-        any_popular = __syncthreads_or(any_popular);
-    }
-
     const int lane = threadIdx.x % G;
     const int worker = blockIdx.x * (pair_block(SR) / G) + threadIdx.x / G;
     if (worker >= a.num_workers) return;
@@ -473,32 +459,18 @@ __global__ void __launch_bounds__(pair_block(SR), pair_min_blocks(SR, HOT)) sgd_
         cp_async_wait_all();
         __syncwarp(gmask);
 
-        // Bit j of hp (hq): the user (item) of record j of chunk t is popular.
-        auto popular = [&](int t, uint32_t &hp, uint32_t &hq) {
-            hp = hq = 0;
-            if (!HOT || !any_popular) return;
-            const int shift = threadIdx.x & 31 & ~(G - 1);
-            const uint32_t group = (G == 32) ? 0xffffffffu : (1u << G) - 1u;
-#pragma unroll
-            for (int i = 0; i < kChunk / G; ++i) {
-                const uint32_t *w = rec + (t & 1) * CW + 3 * (lane + i * G);
-                const uint32_t h = popular_hash(w[0]), g = popular_hash(w[1]);
-                hp |= ((__ballot_sync(gmask, (s_popular[0][h >> 5] >> (h & 31)) & 1u) >> shift) & group) << (i * G);
-                hq |= ((__ballot_sync(gmask, (s_popular[1][g >> 5] >> (g & 31)) & 1u) >> shift) & group) << (i * G);
-            }
-        };
         // One record on its own: rows p and q become the updated ones, and are stored.
-        auto apply = [&](uint4 &p, uint4 &q, uint32_t uu, uint32_t vv, float r, uint32_t x, uint32_t hu, uint32_t hv) {
+        auto apply = [&](uint4 &p, uint4 &q, uint32_t uu, uint32_t vv, float r, uint32_t x) {
             float s = dot_word<KIND>(p, q, 0.f);
 #pragma unroll
             for (int o = G / 2; o >= 1; o >>= 1) s += __shfl_xor_sync(gmask, s, o);
             uint4 wp, wq;
             update_word<KIND, SR>(p, q, wp, wq, lr, r - s, nlp, nlq, SR ? round_key ^ lowbias32(x) : 0u, lane);
             p = wp;
-            store_row(P + (uint64_t)uu * ROW_WORDS, p, pol_row, hu);
-            if (HOT || !a.freeze_q) {
+            st_row_hint(P + (uint64_t)uu * ROW_WORDS, p, pol_row);
+            if (!a.freeze_q) {
                 q = wq;
-                store_row(Q + (uint64_t)vv * ROW_WORDS, q, pol_row, hv);
+                st_row_hint(Q + (uint64_t)vv * ROW_WORDS, q, pol_row);
             }
         };
         uint32_t nu[2], nv[2];  // ids of the next pair
@@ -507,8 +479,6 @@ __global__ void __launch_bounds__(pair_block(SR), pair_min_blocks(SR, HOT)) sgd_
             nu[e] = rec[3 * e];
             nv[e] = rec[3 * e + 1];
         }
-        uint32_t hp, hq;
-        popular(0, hp, hq);
 
         for (int t = 0; t < chunks; ++t) {
             __syncwarp(gmask);  // the half refilled next is no longer read
@@ -517,7 +487,7 @@ __global__ void __launch_bounds__(pair_block(SR), pair_min_blocks(SR, HOT)) sgd_
             const int next_half = (t & 1) ? -2 * CW : 0;  // added to an index past this chunk's end
 
 #pragma unroll 1
-            for (int j = 0; j < kChunk; j += 2, hp >>= 2, hq >>= 2) {
+            for (int j = 0; j < kChunk; j += 2) {
                 const uint32_t ua = nu[0], ub = nu[1], va = nv[0], vb = nv[1];
                 // Ids outside the matrices load the last row instead; such records are not applied.
                 uint4 *const pa = P + (uint64_t)min(ua, m1) * ROW_WORDS, *const qa = Q + (uint64_t)min(va, n1) * ROW_WORDS;
@@ -555,37 +525,22 @@ __global__ void __launch_bounds__(pair_block(SR), pair_min_blocks(SR, HOT)) sgd_
                     uint4 wpa, wqa, wpb, wqb;
                     update_word<KIND, SR>(fpa, fqa, wpa, wqa, lr, ra - sa, nlp, nlq, SR ? round_key ^ lowbias32(x) : 0u,
                                           lane);
-                    if (!HOT) {
-                        st_row_hint(pa, wpa, pol_row);
-                        if (!a.freeze_q) st_row_hint(qa, wqa, pol_row);
-                    }
+                    st_row_hint(pa, wpa, pol_row);
+                    if (!a.freeze_q) st_row_hint(qa, wqa, pol_row);
                     update_word<KIND, SR>(fpb, fqb, wpb, wqb, lr, rb - sb, nlp, nlq,
                                           SR ? round_key ^ lowbias32(x + 1u) : 0u, lane);
-                    if (!HOT) {
-                        st_row_hint(pb, wpb, pol_row);
-                        if (!a.freeze_q) st_row_hint(qb, wqb, pol_row);
-                    } else if (__builtin_expect(((hp | hq) & 3u) == 0, 1)) {
-                        st_row_hint(pa, wpa, pol_row);
-                        st_row_hint(qa, wqa, pol_row);
-                        st_row_hint(pb, wpb, pol_row);
-                        st_row_hint(qb, wqb, pol_row);
-                    } else {
-                        store_row(pa, wpa, pol_row, hp & 1u);
-                        store_row(qa, wqa, pol_row, hq & 1u);
-                        store_row(pb, wpb, pol_row, hp & 2u);
-                        store_row(qb, wqb, pol_row, hq & 2u);
-                    }
+                    st_row_hint(pb, wpb, pol_row);
+                    if (!a.freeze_q) st_row_hint(qb, wqb, pol_row);
                 } else {
                     if (oka) {
-                        apply(fpa, fqa, ua, va, ra, x, hp & 1u, hq & 1u);
+                        apply(fpa, fqa, ua, va, ra, x);
                         if (ub == ua) fpb = fpa;
                         if (vb == va) fqb = fqa;
                     }
-                    if (okb) apply(fpb, fqb, ub, vb, rb, x + 1u, hp & 2u, hq & 2u);
+                    if (okb) apply(fpb, fqb, ub, vb, rb, x + 1u);
                     if (!(oka & okb)) bad = 1;
                 }
             }
-            popular(t + 1, hp, hq);  // (past the last chunk: old records, not used)
         }
     }
     if (bad && a.status != nullptr && lane == 0) atomicExch(a.status, (int)CUMF_ERR_RANGE);
@@ -790,21 +745,20 @@ using KernelFn = void (*)(const UpdateArgs);
 struct KernelEntry {
     int k, kind, lanes;
     bool sr;
-    KernelFn fn;          // sgd_pair_kernel, or sgd_hogwild_kernel where a lane holds several words
-    KernelFn hot;         // sgd_pair_kernel with popular rows told apart (nullptr otherwise)
+    KernelFn fn;          // sgd_hogwild_kernel
+    KernelFn pair;        // sgd_pair_kernel (nullptr where a lane holds several words)
     KernelFn ring;        // deeper-pipeline variant (nullptr where not built)
     size_t ring_smem;     // its dynamic shared memory per block
 };
 
-// The kernel of a lane width: two records at a time where a lane holds one 16-byte word of a row.
-template <int K, int KIND, int G, bool SR, bool HOT>
-constexpr KernelFn update_kernel() {
-    if constexpr (K * store_bytes(KIND) / 16 == G) return &sgd_pair_kernel<K, KIND, G, SR, HOT>;
-    else return HOT ? nullptr : &sgd_hogwild_kernel<K, KIND, G, SR>;
+template <int K, int KIND, int G, bool SR>
+constexpr KernelFn pair_kernel() {
+    if constexpr (K * store_bytes(KIND) / 16 == G) return &sgd_pair_kernel<K, KIND, G, SR>;
+    else return nullptr;
 }
 
-#define CUMF_K(K, KIND, G, SR) {K, KIND, G, SR, update_kernel<K, KIND, G, SR, false>(), \
-    update_kernel<K, KIND, G, SR, true>(), &sgd_ring_kernel<K, KIND, G, SR, kRingDepth>, RingLayout<K, KIND, G, kRingDepth>::smem}
+#define CUMF_K(K, KIND, G, SR) {K, KIND, G, SR, &sgd_hogwild_kernel<K, KIND, G, SR>, pair_kernel<K, KIND, G, SR>(), \
+    &sgd_ring_kernel<K, KIND, G, SR, kRingDepth>, RingLayout<K, KIND, G, kRingDepth>::smem}
 #define CUMF_K_ALL_G(K, KIND, SR, G1, G2) CUMF_K(K, KIND, G1, SR), CUMF_K(K, KIND, G2, SR)
 
 // For each (k, storage) two lane widths: one 16-byte word per lane, or two.
@@ -869,10 +823,15 @@ static cudaError_t prepare_ring(const KernelEntry *e) {
 int resident_workers(int k, int precision, int lanes, int sm_count) {
     const KernelEntry *e = find_kernel(k, precision, lanes);
     if (!e) return 0;
-    const int threads = e->hot ? pair_block(e->sr) : kBlock;
     int blocks = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, e->fn, threads, 0) != cudaSuccess) return 0;
-    return blocks * sm_count * (threads / e->lanes);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, e->fn, kBlock, 0) != cudaSuccess) return 0;
+    int threads = blocks * kBlock;
+    if (e->pair) {  // either kernel may run (launch_sgd_update)
+        const int t = pair_block(e->sr);
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, e->pair, t, 0) != cudaSuccess) return 0;
+        threads = std::min(threads, blocks * t);
+    }
+    return threads / e->lanes * sm_count;
 }
 
 int wave_workers(int k, int precision, int lanes, int sm_count) {
@@ -907,7 +866,7 @@ cudaError_t launch_sgd_update(const cumf_node *d_R, int64_t nnz, void *d_P, int3
                               void *d_Q, int32_t n, int k, int precision, int num_workers,
                               const Tuning &tuning, const float *d_lr, int first_epoch,
                               int n_epochs, float lambda_p, float lambda_q, uint64_t seed,
-                              int *d_status, cudaStream_t stream, int *lanes_used) {
+                              int *d_status, cudaStream_t stream, int *lanes_used, void *d_flags) {
     Tuning t = resolve_tuning(k, precision, tuning);
     int dev = 0, l2 = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess ||
@@ -940,13 +899,14 @@ cudaError_t launch_sgd_update(const cumf_node *d_R, int64_t nnz, void *d_P, int3
     a.prefetch = t.prefetch;
     a.hints = t.hints;
     a.freeze_q = t.freeze_q;
-    a.hot = nullptr;
+    a.contended = nullptr;
+    a.run_contended = 0;
     // Every worker has to run an epoch before any runs the next one's learning rate: with more
     // workers than fit, one launch per epoch.
     if (n_epochs > 1 && !t.ring && num_workers > resident_workers(k, precision, e->lanes, sms)) {
         for (int ep = first_epoch; ep < first_epoch + n_epochs; ++ep) {
             const cudaError_t ce = launch_sgd_update(d_R, nnz, d_P, m, d_Q, n, k, precision, num_workers, tuning, d_lr, ep,
-                                                     1, lambda_p, lambda_q, seed, d_status, stream, nullptr);
+                                                     1, lambda_p, lambda_q, seed, d_status, stream, nullptr, d_flags);
             if (ce != cudaSuccess) return ce;
         }
         return cudaSuccess;
@@ -958,35 +918,37 @@ cudaError_t launch_sgd_update(const cumf_node *d_R, int64_t nnz, void *d_P, int3
         e->ring<<<(num_workers + gpb - 1) / gpb, kBlock, e->ring_smem, stream>>>(a);
         return cudaGetLastError();
     }
-    const int threads = e->hot ? pair_block(e->sr) : kBlock, gpb = threads / e->lanes;
-    // Row copies have no popular rows, and frozen item rows are not stored.  Under stream capture
-    // (and when no scratch can be had) every store is plain.
-    void *popular = nullptr;
-    const int64_t in_flight = 2ll * std::min(num_workers, threads * pair_min_blocks(e->sr, true) / e->lanes * sms);
+    auto launch = [&](bool pair, const uint2 *contended) {
+        const int threads = pair ? pair_block(e->sr) : kBlock, gpb = threads / e->lanes;
+        a.contended = contended;
+        a.run_contended = pair ? 0 : 1;
+        (pair ? e->pair : e->fn)<<<(num_workers + gpb - 1) / gpb, threads, 0, stream>>>(a);
+        return cudaGetLastError();
+    };
+    if (!e->pair) return launch(false, nullptr);
+    // A copied row has few workers by its plan; and no row is named by more records than there are.
+    const int wave = pair_block(e->sr) * pair_min_blocks(e->sr) / e->lanes * sms;
+    const int64_t in_flight = 2ll * std::min(num_workers, wave);
+    const int limit = contended_limit(k * elem_bytes(precision), e->sr);
+    if (tuning.copies || in_flight <= limit) return launch(true, nullptr);
+    // One record at a time also where that cannot be sampled: too few hits, no scratch, or a
+    // stream capture (its replays may meet other ratings).
+    const int samples = (int)std::min<int64_t>((kLimitHits * in_flight + limit - 1) / limit, kMaxSamples);
+    const int64_t hits = (int64_t)samples * limit / in_flight;
+    void *flags = d_flags;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (e->hot && !tuning.copies && !t.freeze_q && in_flight >= popular_min_in_flight(e->sr)) {
-        if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
-            scratch_alloc(&popular, 2 * kPopularWords * sizeof(uint32_t), stream) != cudaSuccess) {
-            cudaGetLastError();
-            popular = nullptr;
-        }
+    if (hits < kMinHits || cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
+        (flags == nullptr && scratch_alloc(&flags, sizeof(uint2), stream) != cudaSuccess)) {
+        cudaGetLastError();
+        return launch(false, nullptr);
     }
-    if (popular) {
-        const int samples = (int)std::min<int64_t>(2 * in_flight, kMaxSamples);
-        // Well above the hits of the unpopular ids that share a hashed id, too.
-        const int64_t limit = std::max<int64_t>((int64_t)kPopularWorkers * samples / in_flight,
-                                                2 + 4ll * samples / (1 << kPopularBits));
-        sample_popular_kernel<<<2, kSampleThreads, 0, stream>>>(d_R, a.nnz, a.m, a.n, samples, (uint32_t)limit,
-                                                                splitmix64(seed), static_cast<uint32_t *>(popular));
-    }
-    a.hot = static_cast<const uint32_t *>(popular);
-    (popular ? e->hot : e->fn)<<<(num_workers + gpb - 1) / gpb, threads, 0, stream>>>(a);
+    sample_rows_kernel<<<2, kSampleThreads, 0, stream>>>(d_R, a.nnz, a.m, t.freeze_q ? 0 : a.n, samples,
+                                                         (uint32_t)(hits + 1), splitmix64(seed), static_cast<uint32_t *>(flags));
     cudaError_t ce = cudaGetLastError();
-    if (popular) {
-        const cudaError_t ef = cudaFreeAsync(popular, stream);
-        if (ce == cudaSuccess) ce = ef;
-    }
-    return ce;
+    if (ce == cudaSuccess) ce = launch(false, static_cast<const uint2 *>(flags));
+    if (ce == cudaSuccess) ce = launch(true, static_cast<const uint2 *>(flags));
+    const cudaError_t ef = flags == d_flags ? cudaSuccess : cudaFreeAsync(flags, stream);
+    return ce == cudaSuccess ? ef : ce;
 }
 
 }  // namespace cumf

@@ -285,7 +285,7 @@ int stream_train(const cumf_problem *tr, const cumf_params &p, int workers, int 
     DevBuf d_lr, d_status;
     CUMF_CUDA(d_lr.alloc(lr.size() * sizeof(float)));
     CUMF_CUDA(cudaMemcpy(d_lr.p, lr.data(), lr.size() * sizeof(float), cudaMemcpyHostToDevice));
-    CUMF_CUDA(d_status.alloc(sizeof(int)));
+    CUMF_CUDA(d_status.alloc(4 * sizeof(int)));  // the status, and at 8 the update launches' flags
     CUMF_CUDA(cudaMemset(d_status.p, 0, sizeof(int)));
 
     int64_t max_grid = 0;
@@ -329,7 +329,7 @@ int stream_train(const cumf_problem *tr, const cumf_params &p, int workers, int 
             CUMF_CUDA(launch_sgd_update(Rc.slot[jr].buf.as<cumf_node>(), grid_size[sp.g], Pc.slot[jp].buf.p,
                                         (int32_t)u_seg, Qc.slot[jq].buf.p, (int32_t)v_seg, k, p.precision, workers,
                                         tu, d_lr.as<float>(), it, 1, lambda_p, lambda_q, block_seed(p.seed, sp.g),
-                                        d_status.as<int>(), comp.s, nullptr));
+                                        d_status.as<int>(), comp.s, nullptr, d_status.as<int>() + 2));
             CUMF_CUDA(cudaEventRecord(Rc.slot[jr].idle, comp.s));
             CUMF_CUDA(cudaEventRecord(Pc.slot[jp].idle, comp.s));
             CUMF_CUDA(cudaEventRecord(Qc.slot[jq].idle, comp.s));

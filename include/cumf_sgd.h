@@ -121,8 +121,8 @@ typedef struct cumf_params {
 typedef struct cumf_tuning {
     int32_t lanes;         /* lanes per rating: 0 = default for (k, precision)           */
     int32_t prefetch;      /* rows of record j+prefetch are pulled into L2 during record j
-                              (two records ahead for any value above 0 where a lane holds one
-                              16-byte word of a row); -1 = default (2; see rows_copied),
+                              (two records ahead for any value above 0 where the launch takes
+                              two records at a time); -1 = default (2; see rows_copied),
                               0 = off, at most 15                                         */
     int32_t l2_hints;      /* -1 = default, 0 = none, 1 = ratings evict_first and factor
                               rows evict_last                                            */
