@@ -295,7 +295,8 @@ batch_kernel(const BatchProblemDev *probs, const BatchTask *tasks, int tasks_per
                 bad = 1;
         }
     }
-    if (bad && status && lane == 0) atomicExch(status, (int)CUMF_ERR_RANGE);
+    // (Only the half of the lanes whose record it was has seen a bad one.)
+    if (__any_sync(gmask, bad) && status && lane == 0) atomicExch(status, (int)CUMF_ERR_RANGE);
 }
 
 }  // namespace
