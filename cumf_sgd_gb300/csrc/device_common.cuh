@@ -146,8 +146,8 @@ __device__ __forceinline__ float dot_word(const uint4 &p, const uint4 &q, float 
 __device__ __forceinline__ float2 both(float x) { return make_float2(x, x); }
 
 // update_rows for one word, two elements per instruction; nlp = -lambda_p, nlq = -lambda_q
-// (-(l*x) and (-l)*x are the same bits).
-template <int KIND, bool SR>
+// (-(l*x) and (-l)*x are the same bits).  kUpdateQ = false: neither q's arithmetic nor its random bits.
+template <int KIND, bool SR, bool kUpdateQ = true>
 __device__ __forceinline__ void update_word(const uint4 &p, const uint4 &q, uint4 &wp, uint4 &wq, float lr, float err,
                                             float nlp, float nlq, uint32_t key, int lane) {
     using C = Conv<KIND>;
@@ -155,14 +155,13 @@ __device__ __forceinline__ void update_word(const uint4 &p, const uint4 &q, uint
     for (int h = 0; h < C::kPairs; ++h) {
         const float2 pp = C::get(p, h), qq = C::get(q, h);
         const float2 a = __ffma2_rn(both(lr), __ffma2_rn(both(err), qq, __fmul2_rn(both(nlp), pp)), pp);
-        const float2 b = __ffma2_rn(both(lr), __ffma2_rn(both(err), pp, __fmul2_rn(both(nlq), qq)), qq);
-        if (SR) {
-            const uint32_t pair = (uint32_t)((lane * C::kPairs + h) * 2);
-            C::put_sr(wp, h, a.x, a.y, lowbias32(key + pair));
-            C::put_sr(wq, h, b.x, b.y, lowbias32(key + pair + 1u));
-        } else {
-            C::put(wp, h, a.x, a.y);
-            C::put(wq, h, b.x, b.y);
+        const uint32_t pair = (uint32_t)((lane * C::kPairs + h) * 2);
+        if (SR) C::put_sr(wp, h, a.x, a.y, lowbias32(key + pair));
+        else C::put(wp, h, a.x, a.y);
+        if (kUpdateQ) {
+            const float2 b = __ffma2_rn(both(lr), __ffma2_rn(both(err), pp, __fmul2_rn(both(nlq), qq)), qq);
+            if (SR) C::put_sr(wq, h, b.x, b.y, lowbias32(key + pair + 1u));
+            else C::put(wq, h, b.x, b.y);
         }
     }
 }

@@ -398,7 +398,11 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(const cumf_
     if (threadIdx.x == 0) flags[blockIdx.x] = over != 0;
 }
 
-template <int K, int KIND, int G, bool SR>
+// FROZEN: a.freeze_q is set, and neither q's arithmetic nor its random bits are computed (a kernel of
+// its own: the choice within the kernel cost the others a sixth of their time, 5,000 x 2,000,
+// 400,000 ratings, fp16-SR, k = 64 0.70 -> 0.82 ms).  5.2M ratings, 50,000 users, k = 128, bf16-SR:
+// 0.76 ms with q computed, 0.57 so; without stochastic rounding q's arithmetic hides.
+template <int K, int KIND, int G, bool SR, bool FROZEN>
 __global__ void __launch_bounds__(pair_block(SR), pair_min_blocks(SR)) sgd_pair_kernel(const UpdateArgs a) {
     if (skip_launch(a)) return;
     constexpr int ROW_WORDS = K * store_bytes(KIND) / 16;
@@ -465,10 +469,10 @@ __global__ void __launch_bounds__(pair_block(SR), pair_min_blocks(SR)) sgd_pair_
 #pragma unroll
             for (int o = G / 2; o >= 1; o >>= 1) s += __shfl_xor_sync(gmask, s, o);
             uint4 wp, wq;
-            update_word<KIND, SR>(p, q, wp, wq, lr, r - s, nlp, nlq, SR ? round_key ^ lowbias32(x) : 0u, lane);
+            update_word<KIND, SR, !FROZEN>(p, q, wp, wq, lr, r - s, nlp, nlq, SR ? round_key ^ lowbias32(x) : 0u, lane);
             p = wp;
             st_row_hint(P + (uint64_t)uu * ROW_WORDS, p, pol_row);
-            if (!a.freeze_q) {
+            if (!FROZEN && !a.freeze_q) {
                 q = wq;
                 st_row_hint(Q + (uint64_t)vv * ROW_WORDS, q, pol_row);
             }
@@ -523,14 +527,14 @@ __global__ void __launch_bounds__(pair_block(SR), pair_min_blocks(SR)) sgd_pair_
                         sb += __shfl_xor_sync(gmask, sb, o);
                     }
                     uint4 wpa, wqa, wpb, wqb;
-                    update_word<KIND, SR>(fpa, fqa, wpa, wqa, lr, ra - sa, nlp, nlq, SR ? round_key ^ lowbias32(x) : 0u,
-                                          lane);
+                    update_word<KIND, SR, !FROZEN>(fpa, fqa, wpa, wqa, lr, ra - sa, nlp, nlq,
+                                                   SR ? round_key ^ lowbias32(x) : 0u, lane);
                     st_row_hint(pa, wpa, pol_row);
-                    if (!a.freeze_q) st_row_hint(qa, wqa, pol_row);
-                    update_word<KIND, SR>(fpb, fqb, wpb, wqb, lr, rb - sb, nlp, nlq,
-                                          SR ? round_key ^ lowbias32(x + 1u) : 0u, lane);
+                    if (!FROZEN && !a.freeze_q) st_row_hint(qa, wqa, pol_row);
+                    update_word<KIND, SR, !FROZEN>(fpb, fqb, wpb, wqb, lr, rb - sb, nlp, nlq,
+                                                   SR ? round_key ^ lowbias32(x + 1u) : 0u, lane);
                     st_row_hint(pb, wpb, pol_row);
-                    if (!a.freeze_q) st_row_hint(qb, wqb, pol_row);
+                    if (!FROZEN && !a.freeze_q) st_row_hint(qb, wqb, pol_row);
                 } else {
                     if (oka) {
                         apply(fpa, fqa, ua, va, ra, x);
@@ -747,18 +751,19 @@ struct KernelEntry {
     bool sr;
     KernelFn fn;          // sgd_hogwild_kernel
     KernelFn pair;        // sgd_pair_kernel (nullptr where a lane holds several words)
+    KernelFn frozen;      // the same with item rows frozen
     KernelFn ring;        // deeper-pipeline variant (nullptr where not built)
     size_t ring_smem;     // its dynamic shared memory per block
 };
 
-template <int K, int KIND, int G, bool SR>
+template <int K, int KIND, int G, bool SR, bool FROZEN>
 constexpr KernelFn pair_kernel() {
-    if constexpr (K * store_bytes(KIND) / 16 == G) return &sgd_pair_kernel<K, KIND, G, SR>;
+    if constexpr (K * store_bytes(KIND) / 16 == G) return &sgd_pair_kernel<K, KIND, G, SR, FROZEN>;
     else return nullptr;
 }
 
-#define CUMF_K(K, KIND, G, SR) {K, KIND, G, SR, &sgd_hogwild_kernel<K, KIND, G, SR>, pair_kernel<K, KIND, G, SR>(), \
-    &sgd_ring_kernel<K, KIND, G, SR, kRingDepth>, RingLayout<K, KIND, G, kRingDepth>::smem}
+#define CUMF_K(K, KIND, G, SR) {K, KIND, G, SR, &sgd_hogwild_kernel<K, KIND, G, SR>, pair_kernel<K, KIND, G, SR, false>(), \
+    pair_kernel<K, KIND, G, SR, SR>(), &sgd_ring_kernel<K, KIND, G, SR, kRingDepth>, RingLayout<K, KIND, G, kRingDepth>::smem}
 #define CUMF_K_ALL_G(K, KIND, SR, G1, G2) CUMF_K(K, KIND, G1, SR), CUMF_K(K, KIND, G2, SR)
 
 // For each (k, storage) two lane widths: one 16-byte word per lane, or two.
@@ -828,8 +833,10 @@ int resident_workers(int k, int precision, int lanes, int sm_count) {
     int threads = blocks * kBlock;
     if (e->pair) {  // either kernel may run (launch_sgd_update)
         const int t = pair_block(e->sr);
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, e->pair, t, 0) != cudaSuccess) return 0;
-        threads = std::min(threads, blocks * t);
+        for (KernelFn fn : {e->pair, e->frozen}) {
+            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fn, t, 0) != cudaSuccess) return 0;
+            threads = std::min(threads, blocks * t);
+        }
     }
     return threads / e->lanes * sm_count;
 }
@@ -922,7 +929,7 @@ cudaError_t launch_sgd_update(const cumf_node *d_R, int64_t nnz, void *d_P, int3
         const int threads = pair ? pair_block(e->sr) : kBlock, gpb = threads / e->lanes;
         a.contended = contended;
         a.run_contended = pair ? 0 : 1;
-        (pair ? e->pair : e->fn)<<<(num_workers + gpb - 1) / gpb, threads, 0, stream>>>(a);
+        (!pair ? e->fn : t.freeze_q ? e->frozen : e->pair)<<<(num_workers + gpb - 1) / gpb, threads, 0, stream>>>(a);
         return cudaGetLastError();
     };
     if (!e->pair) return launch(false, nullptr);
