@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "cumf_sgd.h"
+#include "index_walk.h"
 #include "internal.h"
 #include "rng.h"
 #include "tc_gemm.h"
@@ -84,12 +85,12 @@ __global__ void user_qsum_kernel(const cumf_node *R, int64_t nnz, int32_t m, int
 // them in order instead of gathering the records.
 __global__ void user_keys_kernel(const cumf_node *R, uint32_t nnz, int32_t m, int32_t n, uint32_t *key,
                                  float2 *val) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += gridDim.x * blockDim.x) {
+    index_walk(blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, nnz, [&](uint32_t i) {
         const cumf_node x = R[i];
         const bool ok = (uint32_t)x.u < (uint32_t)m && (uint32_t)x.v < (uint32_t)n;
         key[i] = ok ? (uint32_t)x.u : (uint32_t)m;
         val[i] = make_float2(x.r, __int_as_float(x.v));
-    }
+    });
 }
 
 // seg[u] = the first sorted position whose key is >= u, u = 0..m (binary search).
@@ -143,12 +144,11 @@ __global__ void __launch_bounds__(kT) user_rows_kernel(const float2 *val, const 
         const uint32_t cnt = (uint32_t)(seg[u + 1] - a);
         const float2 *row = val + a;
         float s = 0.f, s2 = 0.f;
-#pragma unroll 4
-        for (uint32_t t = lane; t < cnt; t += 32) {
+        index_walk<4>(lane, 32, cnt, [&](uint32_t t) {
             const float r = row[t].x;
             s += r;
             s2 += r * r;
-        }
+        });
         for (int o = 16; o >= 1; o >>= 1) {
             s += __shfl_xor_sync(0xffffffffu, s, o);
             s2 += __shfl_xor_sync(0xffffffffu, s2, o);
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(kT) user_rows_kernel(const float2 *val, const 
             }
             float2 next = make_float2(0.f, 0.f);
             if ((uint32_t)lane < cnt) next = row[lane];
-            for (uint32_t t0 = 0; t0 < cnt; t0 += 32) {
+            index_walk(0, 32, cnt, [&](uint32_t t0) {
                 const float c = (next.x - s / d) / d;
                 const int item = __float_as_int(next.y);
                 if (cnt - t0 > 32 + (uint32_t)lane) next = row[t0 + 32 + lane];
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(kT) user_rows_kernel(const float2 *val, const 
                         for (int j = 0; j < V; ++j) acc[g][j] += c4[0] * q[0][g][j];
                     }
                 }
-            }
+            });
 #pragma unroll
             for (int g = 0; g < G; ++g)
                 if (cl + g * 32 * V < k) {
