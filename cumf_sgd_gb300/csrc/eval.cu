@@ -635,22 +635,21 @@ extern "C" int cumf_evaluate(const cumf_problem *te, const cumf_model *model, in
     if ((te->nnz > 0 && !te->R) || (!model->P && model->m > 0) || (!model->Q && model->n > 0) || model->k <= 0)
         return fail(CUMF_ERR_ARG, "evaluate: malformed input");
     if (int rc = select_device(0)) return rc;
+    if (te->nnz == 0) {
+        *out = NAN;  // 0 / 0 (mf.cpp:4029-4030)
+        return CUMF_OK;
+    }
     Stream stream;
     CUMF_CUDA(cudaStreamCreateWithFlags(&stream.s, cudaStreamNonBlocking));
     DevBuf d_R, d_P, d_Q, d_part, d_sum;
     const size_t pb = (size_t)model->m * model->k * sizeof(float), qb = (size_t)model->n * model->k * sizeof(float);
-    CUMF_CUDA(d_R.alloc(std::max<int64_t>(1, te->nnz) * sizeof(cumf_node), stream.s));
+    CUMF_CUDA(d_R.alloc(te->nnz * sizeof(cumf_node), stream.s));
     CUMF_CUDA(d_P.alloc(pb, stream.s));
     CUMF_CUDA(d_Q.alloc(qb, stream.s));
-    if (te->nnz)
-        CUMF_CUDA(cudaMemcpyAsync(d_R.p, te->R, te->nnz * sizeof(cumf_node), cudaMemcpyHostToDevice, stream.s));
+    CUMF_CUDA(cudaMemcpyAsync(d_R.p, te->R, te->nnz * sizeof(cumf_node), cudaMemcpyHostToDevice, stream.s));
     if (pb) CUMF_CUDA(cudaMemcpyAsync(d_P.p, model->P, pb, cudaMemcpyHostToDevice, stream.s));
     if (qb) CUMF_CUDA(cudaMemcpyAsync(d_Q.p, model->Q, qb, cudaMemcpyHostToDevice, stream.s));
     if (ranking) {
-        if (te->nnz == 0) {
-            *out = NAN;  // 0 / 0 (mf.cpp:4029-4030)
-            return CUMF_OK;
-        }
         double two[2] = {0, 0};
         const int transpose = (criterion == kColMPR || criterion == kColAUC);
         if (int rc = mpr_auc_device(d_R.as<cumf_node>(), te->nnz, te->m, te->n, d_P.as<float>(), model->m,

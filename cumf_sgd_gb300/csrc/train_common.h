@@ -52,10 +52,14 @@ struct DevBuf {
     }
 };
 
+// A call's own stream.  It is waited for at the end, since buffers freed on it (DevBuf) wait for nothing:
+// a call that fails may have copies from the caller's memory in flight (otherwise it is idle by then).
 struct Stream {
     cudaStream_t s = nullptr;
     ~Stream() {
-        if (s) cudaStreamDestroy(s);
+        if (!s) return;
+        cudaStreamSynchronize(s);
+        cudaStreamDestroy(s);
     }
 };
 
