@@ -587,7 +587,9 @@ int mpr_auc_device(const cumf_node *d_R, int64_t nnz, int32_t prob_m, int32_t pr
             transpose_f32_kernel<<<tg, dim3(32, 8), 0, s>>>(Cf, cf_rows, k, cfT.as<float>());
         }
         const size_t factors = (size_t)kRowsPerSweep * k * sizeof(float);
-        const int pred_cap = factors <= 200 * 1024 ? kSweepPreds : 0;  // (long rows of factors leave no room)
+        // Long rows of factors leave no room.  With a constant that is not a number, predictions may be
+        // none either, and what a search then finds depends on its steps: the general one's.
+        const int pred_cap = factors <= 200 * 1024 && !std::isnan(b) ? kSweepPreds : 0;
         const size_t smem = factors + pred_cap * sizeof(float);
         if (smem > 46 * 1024)  // with the static arrays, more than the default 48 KB
             CUMF_CUDA(cudaFuncSetAttribute(sweep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
