@@ -255,7 +255,9 @@ __global__ void __launch_bounds__(kT) sweep_kernel(const int64_t *__restrict__ a
     extern __shared__ __align__(16) float s_p[];  // k x kRowsPerSweep row factors, then pred_cap predictions
     float *const s_pred = s_p + kRowsPerSweep * k;
     __shared__ int64_t s_seg[kRowsPerSweep], s_off[kRowsPerSweep], s_len[kRowsPerSweep];
-    __shared__ int s_valid[kRowsPerSweep], s_at[kRowsPerSweep + 1];
+    // (Small types: with these arrays, rows of up to 3,623 factors fit the 227 KB of a block.)
+    __shared__ uint16_t s_at[kRowsPerSweep + 1];
+    __shared__ bool s_valid[kRowsPerSweep];
     __shared__ unsigned long long s_cnt[kRowsPerSweep];
     const int64_t g0 = (int64_t)blockIdx.x * kRowsPerSweep;
     const int nr = (nactive - g0 < kRowsPerSweep) ? (int)(nactive - g0) : kRowsPerSweep;
@@ -279,10 +281,10 @@ __global__ void __launch_bounds__(kT) sweep_kernel(const int64_t *__restrict__ a
     if (threadIdx.x == 0) {
         int64_t at = 0;
         for (int r = 0; r < kRowsPerSweep; ++r) {
-            s_at[r] = (int)min(at, (int64_t)pred_cap + 1);
+            s_at[r] = (uint16_t)min(at, (int64_t)pred_cap + 1);
             at += s_len[r];
         }
-        s_at[kRowsPerSweep] = (int)min(at, (int64_t)pred_cap + 1);
+        s_at[kRowsPerSweep] = (uint16_t)min(at, (int64_t)pred_cap + 1);
     }
     for (int idx = threadIdx.x; idx < kRowsPerSweep * k; idx += blockDim.x) {
         const int r = idx / k, t = idx % k;
