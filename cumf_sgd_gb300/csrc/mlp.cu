@@ -506,17 +506,20 @@ void wgrad_jobs(Mlp *mp, int64_t rp, WgradJob *job) {
 
 // Workspace for batches of up to `rows` rows: the forward buffers, and with `train` also
 // those of the backward pass (the batch's targets, the activations' transposes and slopes, gradients).
+// A capacity is 0 while its buffers are replaced: where one cannot be had, the others have gone.
 int mlp_ensure(Mlp *mp, int64_t rows, bool train) {
     const int64_t r = (rows + 127) / 128 * 128;
     const size_t b2 = 2;
     const int h = mp->h, dp = mp->dp, dout = mp->d_out;
     if (rows > mp->cap_fwd) {
+        mp->cap_fwd = 0;
         CUMF_CUDA(mp->xb.alloc(r * dp * b2));
         CUMF_CUDA(mp->h1.alloc(r * h * b2));
         CUMF_CUDA(mp->h2.alloc(r * h * b2));
         mp->cap_fwd = r;
     }
     if (!train || rows <= mp->cap) return CUMF_OK;
+    mp->cap = 0;
     CUMF_CUDA(mp->tb.alloc(r * dout * 4));
     CUMF_CUDA(mp->slope1.alloc(r * h * 4));
     CUMF_CUDA(mp->slope2.alloc(r * h * 4));

@@ -27,16 +27,14 @@ struct DevBuf {
     cudaError_t alloc(size_t b) {
         release();
         bytes = b;
-        return cudaMalloc(&p, b ? b : 16);
+        return checked(cudaMalloc(&p, b ? b : 16));
     }
     cudaError_t alloc(size_t b, cudaStream_t stream) {
         release();
         bytes = b;
-        const cudaError_t e = scratch_alloc(&p, b ? b : 16, stream);
-        if (e != cudaSuccess) p = nullptr;
         pooled = true;
         s = stream;
-        return e;
+        return checked(scratch_alloc(&p, b ? b : 16, stream));
     }
     template <typename T>
     T *as() const { return reinterpret_cast<T *>(p); }
@@ -44,6 +42,13 @@ struct DevBuf {
   private:
     cudaStream_t s = nullptr;
     bool pooled = false;
+    // Without memory: no buffer, and no error left for the next launch to find.
+    cudaError_t checked(cudaError_t e) {
+        if (e == cudaSuccess) return e;
+        p = nullptr;
+        cudaGetLastError();
+        return e;
+    }
     void release() {
         if (p && pooled) cudaFreeAsync(p, s);
         else if (p) cudaFree(p);

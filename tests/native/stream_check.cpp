@@ -11,6 +11,7 @@ static int freed;
 
 extern "C" {
 cudaError_t cudaMalloc(void **p, size_t) { return *p = &freed, cudaSuccess; }
+cudaError_t cudaGetLastError(void) { return cudaSuccess; }
 cudaError_t cudaFree(void *) { return calls += "free ", cudaSuccess; }
 cudaError_t cudaFreeAsync(void *, cudaStream_t s) { return calls += s ? "free-on-stream " : "free-on-null ", cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return calls += "wait ", cudaSuccess; }
