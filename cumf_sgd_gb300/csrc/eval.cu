@@ -603,7 +603,7 @@ int mpr_auc_device(const cumf_node *d_R, int64_t nnz, int32_t prob_m, int32_t pr
                                                         segcnt.as<unsigned long long>());
         CUMF_CUDA(cudaGetLastError());
     }
-    // 5. row terms, summed in row order.
+    // 5. row terms, summed in a fixed order.
     CUMF_CUDA(mpr.alloc(nseg * 8, s));
     CUMF_CUDA(auc.alloc(nseg * 8, s));
     CUMF_CUDA(posb.alloc(nseg * 8, s));

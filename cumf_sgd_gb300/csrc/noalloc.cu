@@ -1,6 +1,6 @@
 // noalloc.cu - an RMSE entry point that allocates no memory.
 //
-// cumf_dev_rmse gets its per-block partial sums from cudaMalloc.  Some callers cannot
+// cumf_dev_rmse gets its per-block partial sums from the scratch pool.  Some callers cannot
 // allocate device memory at the point where they want an evaluation: code running inside a
 // memory pool or arena that must not grow, allocator hooks and out-of-memory handlers, and
 // callers that hand this library only fixed, pre-sized buffers.  For them,

@@ -138,8 +138,9 @@ __global__ void import_kernel(const float *src, const int32_t *map, uint64_t row
 // ratings are fetched while these are summed, a group takes U ratings at a time where a row is
 // short (k = 32 C, C loads per lane and row; C = 0: any k, one at a time), and the grid is what
 // is resident at once, 5 blocks on each of 152 SMs: with 1,024 blocks a third of them ran in a
-// second wave.  1.4M ratings, 480,189 x 17,770, k = 128: 154 us, 82 so
-// (79 with 4 blocks of 64 registers, 85 with 6 of 40).
+// second wave (the count is not asked of the device, since the sum's bits depend on it).  1.4M
+// ratings, 480,189 x 17,770, k = 128: 154 us, 82 so (79 with 4 blocks of 64 registers, 85 with 6
+// of 40).
 constexpr int kRmseLanes = 8;
 constexpr int kRmsePerSm = 5;
 constexpr int kRmseBlocks = kRmsePerSm * 152;

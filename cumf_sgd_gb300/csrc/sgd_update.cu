@@ -326,7 +326,7 @@ sgd_hogwild_kernel(const UpdateArgs a) {
 // many as with one record at a time and the next one's rows in flight.  Loading a pair ahead
 // (four records) is faster still (3,000 x 1,200: 0.25 ms) but loses twice the updates on popular
 // rows: 10,000 x 2,000, 0.9M ratings, Zipf 1.0, 20 epochs, test RMSE 0.8069 at 878 workers and
-// 0.905 at 7,904, against 0.8038 and 0.842 as here (0.8030 and 0.841 one record at a time).
+// 0.905 at 7,904, against 0.8038 and 0.842 so (0.8030 and 0.841 one record at a time).
 // With the GPU full the epoch is bound by L2: what pays there is fewer instructions per record (no
 // zero fill, no register moves, no forwarding; fp16 and bf16 products accumulate by
 // mixed-precision fma, exact as the widened ones; f32x2 pairs in the update).  1024 threads per

@@ -597,7 +597,8 @@ void launch_parse(const unsigned char *t, int64_t start, int64_t len, int64_t nb
                   uint32_t *out_words, unsigned long long cap_tokens, unsigned long long *bad,
                   const unsigned long long *carry, int64_t byte_base, uint32_t *block_flags, cudaStream_t s) {
     parse_tokens_kernel<<<(unsigned)nb, kTB, 0, s>>>(t, start, len, block_base, out_words, cap_tokens, carry, block_flags);
-    parse_rest_kernel<<<(unsigned)std::min<int64_t>(nb, 608), kTB, 0, s>>>(t, start, len, nb, block_base, out_words,
+    // (4 blocks on each of 152 SMs; any number does.)
+    parse_rest_kernel<<<(unsigned)std::min<int64_t>(nb, 4 * 152), kTB, 0, s>>>(t, start, len, nb, block_base, out_words,
                                                                            cap_tokens, bad, carry, byte_base, block_flags);
 }
 

@@ -64,9 +64,9 @@ CUMF_HD uint32_t digits4(uint32_t d) {
     return (d * 100u + (d >> 16)) & 0xffffu;
 }
 
-// Four characters that are all digits: their low halves; *ok is cleared otherwise.  (A byte is a
-// digit iff its high half is 3 and adding 6 leaves it 3; a carry into the next byte comes only
-// from a byte that is none.)
+// Four characters that are all digits: their low halves; *ok is cleared otherwise.  (The test that
+// simdjson's number parser is known for: a byte is a digit iff its high half is 3 and adding 6
+// leaves it 3; a carry into the next byte comes only from a byte that is none.)
 CUMF_HD uint32_t digit_values(uint32_t y, bool *ok) {
     *ok &= ((y & 0xf0f0f0f0u) | (((y + 0x06060606u) & 0xf0f0f0f0u) >> 4)) == 0x33333333u;
     return y & 0x0f0f0f0fu;
